@@ -155,6 +155,64 @@ def run(s):
                                b2=s["b2"])
 
 
+def _dense(codes, scale):
+    """[rows, K / 2] packed codes and [rows, K / 32] exponent bytes -> [rows, K] in 64 bits, by the layer's own table."""
+    table = torch.tensor([0.0, 0.25, 1.0, 1.5, 2.0, 3.0, math.inf, math.nan], dtype=torch.float64, device=codes.device)
+    table = torch.cat([table, -table])
+    v = table[torch.stack([codes & 15, codes >> 4], dim=-1).flatten(-2).long()]
+    return v * torch.exp2(scale.double() - 127.0).repeat_interleave(32, dim=1)
+
+
+def exact(case, seed):
+    """The layer in 64 bits from end to end, nothing rounded in between."""
+    s, T = prepare(case, seed), case["tokens"]
+    x = s["x"].double()
+    layer = s.get("layer")
+    if layer is not None:
+        w13, s13, w2, s2, b13, b2 = layer.w13, layer.w13_scale, layer.w2, layer.w2_scale, None, None
+        logits = x @ layer.router_weight.double().T if s["logits"] is None else s["logits"].double()
+        E, k = logits.shape[1], case["top_k"]
+        if case["routing"] == "softmax":
+            score = torch.softmax(logits, dim=1)
+            weights, ids = score.topk(k, dim=1)
+            weights = weights / weights.sum(1, keepdim=True)
+        else:   # the best four of eight groups by the sum of a group's two largest choices; weights without the bias
+            score = torch.sigmoid(logits)
+            choice = score + layer.router_bias.double()
+            groups = choice.view(T, 8, E // 8)
+            kept = groups.topk(2, dim=2)[0].sum(2).topk(4, dim=1)[1]
+            open_ = torch.zeros(T, 8, dtype=torch.bool, device=x.device).scatter_(1, kept, True)
+            ids = groups.masked_fill(~open_[:, :, None], -math.inf).flatten(1).topk(k, dim=1)[1]
+            weights = score.gather(1, ids)
+            weights = 2.5 * weights / weights.sum(1, keepdim=True)
+        if case["shared"]:
+            ids = torch.cat([ids, torch.full((T, 1), E, device=x.device)], dim=1)
+            weights = torch.cat([weights, torch.ones((T, 1), dtype=torch.float64, device=x.device)], dim=1)
+    else:
+        w13, s13, w2, s2, b13, b2 = (s[n] for n in ("w13", "s13", "w2", "s2", "b13", "b2"))
+        ids, weights = s["ids"].long(), s["weights"].double()
+    out = torch.zeros((T, case["hidden"]), dtype=torch.float64, device=x.device)
+    for e in range(w13.shape[0]):
+        rows, slot = (ids == e).nonzero(as_tuple=True)
+        if rows.numel() == 0:
+            continue
+        h = x[rows] @ _dense(w13[e], s13[e]).T
+        if b13 is not None:
+            h = h + b13[e].double()
+        g, u = h.chunk(2, dim=1)
+        if case["situ"]:
+            a = 4.0 * torch.tanh(g / 4.0) * torch.sigmoid(g) * (25.0 * torch.tanh(u / 25.0))
+        else:
+            if case["limit"] > 0:
+                g, u = g.clamp(max=case["limit"]), u.clamp(-case["limit"], case["limit"])
+            a = g * torch.sigmoid(g) * u
+        y = a @ _dense(w2[e], s2[e]).T
+        if b2 is not None:
+            y = y + b2[e].double()
+        out.index_add_(0, rows, y * weights[rows, slot][:, None])
+    return out
+
+
 def work(case):
     """Weights and scales of the experts the batch is expected to touch, activations in, bf16 result out, and the router
     weight or the given routing; three multiply-add GEMMs per routed slot."""
