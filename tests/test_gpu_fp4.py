@@ -1,0 +1,117 @@
+"""-m gpu: the small-tile fp4 GEMM form at the edges of its tiles - tokens per expert around 8, 16 and 32 (one MMA column
+block of 8 or 16 tokens, two of 16, several tiles), K from a quarter of a stage to several, a ragged last feature tile - and
+with everything its number format has no code for."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from gpu_common import DEV, gpu_layer, oracle_layer, to_np  # noqa: E402
+from helpers import assert_close_bf16  # noqa: E402
+from vkernels_b200 import synthetic as syn  # noqa: E402
+from vkernels_b200 import torch_ops as ops  # noqa: E402
+
+
+def _problem(H, I, counts, seed=3):
+    """Expert e gets counts[e] tokens (top-1); weights, activations, ids, routing weights."""
+    cfg = syn.scaled(syn.CONFIGS["c0"], H=H, I=I, E=len(counts), top_k=1)
+    T = sum(counts)
+    w = syn.make_expert_weights(cfg, seed=seed, device=DEV)
+    A = syn.make_activations(cfg, T, seed=seed, device=DEV)
+    rng = np.random.default_rng(seed)
+    ids = rng.permutation(np.repeat(np.arange(len(counts)), counts)).astype(np.int32)[:, None]
+    tw = (0.5 + rng.random((T, 1))).astype(np.float32)
+    return w, A, torch.from_numpy(ids).to(DEV), torch.from_numpy(tw).to(DEV)
+
+
+def _bf16_forms(w, A, ids, tw, **kw):
+    """Outputs of the bf16-output form from the checkpoint layout and from prepacked weights."""
+    E, I, H, T = w["w13"].shape[0], w["w13"].shape[1] // 2, A.shape[1], A.shape[0]
+    sids, eids, _ = ops.moe_align_block_size(ids, E, 16)
+    act = torch.zeros((sids.numel(), I), dtype=torch.bfloat16, device=DEV)
+    y = [torch.full((T, H), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    args = (tw.reshape(-1).contiguous(), sids, eids)
+    ops.fused_moe_mxfp4_bf16_into(y[0], act, A, w["w13"], w["w13_scale"], w["w2"], w["w2_scale"], *args, top_k=ids.shape[1], **kw)
+    pk = ops.prepack_weights(w["w13"], w["w13_scale"], w["w2"], w["w2_scale"])
+    if pk.usable:
+        ops.fused_moe_mxfp4_bf16_prepacked_into(y[1], act, A, pk, *args, top_k=ids.shape[1], **kw)
+    torch.cuda.synchronize()
+    ops.kernel_status()
+    return to_np(y[0].float()), to_np(y[1].float()) if pk.usable else None
+
+
+@pytest.mark.parametrize("H,I", [(64, 64), (128, 320), (320, 192), (576, 2112)])
+@pytest.mark.parametrize("counts", [(8,) * 2, (1, 0, 9, 3), (16, 7, 17), (31, 32, 33), (0, 70, 1)])
+def test_tile_edges(H, I, counts):
+    w, A, ids, tw = _problem(H, I, counts)
+    w["w13_scale"][0, I + 3, -1] = 0xFF      # a zero group in an up row, one in a down row
+    w["w2_scale"][-1, 7, 0] = 0xFF
+    for kw in ({}, {"activation": 1}, {"swiglu_limit": 0.25}):
+        ref = oracle_layer(A, w, ids, tw, **kw)
+        got = to_np(gpu_layer(A, w, ids, tw, **kw))
+        assert_close_bf16(got, ref, f"fp32 output {H} {I} {counts} {kw}")
+        # The GEMMs are exact to fp32 rounding; what is left is the activation's rounding to bf16 falling the other way
+        # for a few elements: at most one step of 2^-8 each.
+        assert np.linalg.norm(got - ref) <= 2.0 ** -8 * np.linalg.norm(ref)
+        if sum(counts) > 12:                 # (fewer slots take the flat kernels)
+            for y in _bf16_forms(w, A, ids, tw, **kw):
+                assert_close_bf16(y, ref, f"bf16 output {H} {I} {counts} {kw}", got_is_bf16=True)
+
+
+def test_wide_range_rows():
+    """Rows whose elements span far more than the seventeen bits of their integers, and rows near both ends of the
+    bf16 range: the error stays below 2^-17 of the row's largest element times the weights' 1-norm."""
+    H, I, counts = 256, 64, (5, 20, 16)
+    w, A, ids, tw = _problem(H, I, counts)
+    T = A.shape[0]
+    g = torch.Generator(device=DEV)
+    g.manual_seed(1)
+    A *= torch.exp2(torch.randint(-24, 1, A.shape, generator=g, device=DEV).float()).to(torch.bfloat16)
+    A *= torch.exp2(torch.linspace(-120, 20, T, device=DEV)).to(torch.bfloat16)[:, None]
+    sids, eids, _ = ops.moe_align_block_size(ids, len(counts), 16)
+    act = torch.zeros((sids.numel(), I), dtype=torch.bfloat16, device=DEV)
+    y = torch.empty((T, H), dtype=torch.bfloat16, device=DEV)
+    # SiTU with huge beta's is close to the identity on small inputs; large ones saturate: only the gate sums matter here,
+    # so compare the activations with those of the CUDA-core path
+    ops.fused_moe_mxfp4_bf16_into(y, act, A, w["w13"], w["w13_scale"], w["w2"], w["w2_scale"], tw.reshape(-1), sids, eids, top_k=1)
+    _, ref, _, _, _ = gpu_layer(A, w, ids, tw, impl="simt", return_parts=True)
+    real = (sids >= 0) & (sids < T)
+    a, r = act[real].double(), ref[real].double()
+    # relative to the row: activations are about u * g / 2 with both linear in the row's scale
+    scale = r.abs().amax(1, keepdim=True).clamp_min(1e-300)
+    assert ((a - r).abs() / scale).max().item() <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("code", [0x6, 0xE, 0x7])
+@pytest.mark.parametrize("which", ["w13", "w2"])
+def test_lone_nonfinite_codes(code, which):
+    """One inf / NaN code (and one inside a zero group) in otherwise finite weights: the outputs that see it, and no
+    others, are inf or NaN as in the CPU definition."""
+    H, I, counts = 320, 192, (9, 17, 33)
+    w, A, ids, tw = _problem(H, I, counts)
+    A[3] = 0.0                                # inf * 0
+    row, k = (I + 70, 257) if which == "w13" else (130, 100)
+    w[which][1, row, k // 2] = (w[which][1, row, k // 2] & 0x0F) | (code << 4) if k & 1 else (w[which][1, row, k // 2] & 0xF0) | code
+    w[which][2, 5, 0] = (w[which][2, 5, 0] & 0xF0) | code
+    w[which + "_scale"][2, 5, 0] = 0xFF
+    ref = oracle_layer(A, w, ids, tw)
+    assert not np.isfinite(ref).all() and np.isfinite(ref).any()
+    if which == "w13":   # an infinite activation enters the down GEMM as NaN in the fp4 form (VK_MOE_SMALL=bf16 keeps it inf)
+        ref = np.where(np.isinf(ref), np.nan, ref)
+    got = to_np(gpu_layer(A, w, ids, tw))
+    assert_close_bf16(got, ref, f"{which} code {code}")
+    y, packed = _bf16_forms(w, A, ids, tw)
+    assert packed is None
+    assert_close_bf16(y, ref, f"{which} code {code}, bf16 output", got_is_bf16=True)
+
+
+def test_nonfinite_activations_poison_their_token_only():
+    H, I, counts = 320, 192, (9, 17, 33)
+    w, A, ids, tw = _problem(H, I, counts)
+    A[2, 7] = float("nan")
+    A[11, 300] = float("inf")
+    got = to_np(gpu_layer(A, w, ids, tw))
+    bad = np.zeros(A.shape[0], bool)
+    bad[[2, 11]] = True
+    assert np.isnan(got[bad]).all() and np.isfinite(got[~bad]).all()
