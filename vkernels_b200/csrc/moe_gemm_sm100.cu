@@ -156,6 +156,14 @@ struct Barriers {
   float tile_w[kPairMaxTok];
 };
 
+// Tensor maps of the token rows. Pair form: m[i] has boxes of 16 (i + 1) rows x 128 K (two 64-K slices, one after the
+// other in shared memory), so that a stage is one copy per CTA - two with extension rows - whatever the tile: a copy costs
+// its issuing thread 200 clocks and more, and with four to eight boxes of 16 or 64 rows a stage that thread was what the
+// kernel waited for. Lone CTA: m[0] and m[1] have boxes of 16 and 64 rows x 64 K.
+struct TokMaps {
+  CUtensorMap m[8];
+};
+
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
@@ -167,8 +175,7 @@ struct Barriers {
 template <bool GATEUP, int KS, int CTAS>
 __global__ void __launch_bounds__(block_threads(CTAS), 1)
 moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
-                      const __grid_constant__ CUtensorMap tmap_b,
-                      const __grid_constant__ CUtensorMap tmap_b64, const GemmParams p) {
+                      const __grid_constant__ TokMaps tok_maps, const GemmParams p) {
   constexpr int kThreads = block_threads(CTAS);
   constexpr int kAccCols = acc_cols(KS, CTAS);
   constexpr int kACols = KS / 2;                                      // columns of one A slot
@@ -176,7 +183,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
   constexpr int kSubPerW = kWStageK / KS;                             // stages per packed-weight stage
   constexpr int kPieces = KS / 64;                                    // 64-K pieces of a stage
   static_assert(kAStages <= kMaxAStages, "A ring too deep for the barrier arrays");
-  static_assert(CTAS == 1 || KS <= 128, "the CTA-pair form takes 64-K or 128-K stages");
+  static_assert(CTAS == 1 || KS == 128, "the CTA-pair form takes 128-K stages");
   // CTAS == 2: two CTAs of a cluster work on one item - 256 weight rows (128 per CTA, each CTA
   // dequantises its own) against ONE token tile of up to 256 tokens, of which each CTA stages only
   // half. The leader (even) CTA issues cta_group::2 MMAs that read both halves; every CTA keeps
@@ -261,8 +268,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
   const int n_stages = (p.K + KS - 1) / KS;           // pipeline stages per item (last may be short)
   const int pitch = p.K / 32;                         // scale bytes per weight row
   const int n_wrows = GATEUP ? 2 * p.n_feat : p.n_feat;
-  // one 64-K slice of a token stage (this CTA's rows; a pair's MMA N is the tile rounded up to 32)
-  const int slice_bytes = CTAS == 2 ? (((p.max_tok + 31) >> 5) << 4) * 128 : p.max_tok * 128;
+  const int slice_bytes = p.max_tok * 128;            // lone CTA: one 64-K slice of a token stage
 
   if (warp == 0) {
     // ------------------- TMA producer: packed weights + scales ---------------
@@ -341,6 +347,8 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
           const int h0 = min(n32, kPairMainTok) >> 1, h1 = (n32 >> 1) - h0;
           const int row_main = tt.row0 + (int)cta_rank * h0;
           const int row_ext = tt.row0 + 2 * h0 + (int)cta_rank * h1;
+          const CUtensorMap* map0 = &tok_maps.m[(h0 >> 4) - 1];
+          const CUtensorMap* map1 = &tok_maps.m[h1 != 0 ? (h1 >> 4) - 1 : 0];
           for (int st = 0; st < n_stages; ++st) {
             if (!mbar_wait(smem_u32(&bars->stage_done[a.slot]), a.phase ^ 1u, abort_flag, 3, 64)) {
               ok = false;
@@ -348,16 +356,11 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
             }
             const uint32_t bar = smem_u32(&bars->a_full[a.slot]);
             const uint32_t dst = smem_u32(b_smem + a.slot * p.b_stage_bytes);
-            const int n_slices = min(kPieces, (p.K - st * KS) / 64);
-            if (leader) mbar_expect_tx(bar, 2 * (h0 + h1) * 128 * n_slices);
-            for (int sl = 0; sl < n_slices; ++sl) {
-              const uint32_t d = dst + sl * slice_bytes;
-              const int k0 = p.k_base + st * KS + sl * 64;
-              int r = 0;
-              for (; r + 64 <= h0; r += 64) tma_load_2d_pair(d + r * 128, &tmap_b64, k0, row_main + r, bar);
-              for (; r < h0; r += 16) tma_load_2d_pair(d + r * 128, &tmap_b, k0, row_main + r, bar);
-              for (r = 0; r < h1; r += 16) tma_load_2d_pair(d + (h0 + r) * 128, &tmap_b, k0, row_ext + r, bar);
-            }
+            // (a slice past the end of K, or past the shard, is zero fill or other columns: it counts, and no MMA reads it)
+            const int c2 = (p.k_base + st * KS) / 64;
+            if (leader) mbar_expect_tx(bar, 2 * (h0 + h1) * 128 * kPieces);
+            tma_load_3d_pair(dst, map0, 0, row_main, c2, bar);
+            if (h1 != 0) tma_load_3d_pair(dst + kPieces * h0 * 128, map1, 0, row_ext, c2, bar);
             a.advance(kAStages);
           }
         }
@@ -384,9 +387,9 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
           for (int sl = 0; sl < n_slices; ++sl) {
             int r = 0;
             for (; r + 64 <= tt.n_rows; r += 64)
-              tma_load_2d(dst + sl * slice_bytes + r * 128, &tmap_b64, p.k_base + k0 + sl * 64, tt.row0 + r, bar);
+              tma_load_2d(dst + sl * slice_bytes + r * 128, &tok_maps.m[1], p.k_base + k0 + sl * 64, tt.row0 + r, bar);
             for (; r < tt.n_rows; r += 16)
-              tma_load_2d(dst + sl * slice_bytes + r * 128, &tmap_b, p.k_base + k0 + sl * 64, tt.row0 + r, bar);
+              tma_load_2d(dst + sl * slice_bytes + r * 128, &tok_maps.m[0], p.k_base + k0 + sl * 64, tt.row0 + r, bar);
           }
           b.advance(p.b_stages);
         }
@@ -408,7 +411,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
       const uint32_t acc_full_bar = smem_u32(&bars->acc_full);
       const uint32_t a0 = tmem_u + kAccCols;
       const uint64_t desc_first = make_b_desc(smem_u32(b_smem));
-      const uint32_t desc_step = (uint32_t)p.b_stage_bytes >> 4, slice16 = (uint32_t)slice_bytes >> 4;
+      const uint32_t desc_step = (uint32_t)p.b_stage_bytes >> 4;
       uint32_t ready = ready0, done = done0, a_addr = a0, phase = 0;
       uint64_t desc = desc_first;
       int slot = 0;
@@ -417,7 +420,8 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
         const int n32 = (n_rows_u + 31) & ~31;
         const int n_main = min(n32, kPairMainTok), n_ext = n32 - n_main;
         const uint32_t idesc = make_idesc(n_main, 256), idesc_ext = make_idesc(n_ext, 256);
-        const uint32_t ext16 = (uint32_t)(n_main >> 1) * 8u;   // descriptor offset of the extension rows
+        // descriptor distances (16-byte units): slice to slice, main to extension rows
+        const uint32_t slice16 = (uint32_t)(n_main >> 1) * 8u, ext16 = kPieces * slice16, slice16_ext = (uint32_t)(n_ext >> 1) * 8u;
         if (!mbar_wait(smem_u32(&bars->acc_empty), acc_phase ^ 1u, abort_flag, 4)) break;
         tc_fence_after();
         for (int st = 0; st < n_stages; ++st) {
@@ -437,7 +441,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
                   tc_mma_ts_pair(tmem_u, a_addr + sl * 32 + kk * 8, desc + sl * slice16 + kk * 2, idesc, acc);
                   if (n_ext != 0)
                     tc_mma_ts_pair(tmem_u + kPairMainTok, a_addr + sl * 32 + kk * 8,
-                                   desc + ext16 + sl * slice16 + kk * 2, idesc_ext, acc);
+                                   desc + ext16 + sl * slice16_ext + kk * 2, idesc_ext, acc);
                 }
               }
             }
@@ -1053,7 +1057,7 @@ CUtensorMap make_map_nd(const void* ptr, CUtensorMapDataType dt, int elem_bytes,
                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     throw std::runtime_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
-  if (cache.size() >= 64) cache.erase(cache.begin());
+  if (cache.size() >= 256) cache.erase(cache.begin());
   cache.emplace_back(key, m);
   return m;
 }
@@ -1063,6 +1067,22 @@ CUtensorMap make_map(const void* ptr, CUtensorMapDataType dt, int elem_bytes, ui
   const uint64_t dims[2] = {inner, outer}, strides[1] = {pitch_bytes};
   const uint32_t box[2] = {box_inner, box_outer};
   return make_map_nd(ptr, dt, elem_bytes, 2, dims, strides, box);
+}
+
+// Token operand: bf16 rows [EM, K], K a multiple of 64.
+TokMaps token_maps(const void* rows, int K, int EM, bool pair) {
+  TokMaps t{};
+  if (pair) {
+    const uint64_t dims[3] = {64, (uint64_t)EM, (uint64_t)K / 64}, strides[2] = {(uint64_t)K * 2, 128};
+    for (uint32_t i = 0; i < 8; ++i) {
+      const uint32_t box[3] = {64, 16 * (i + 1), 2};
+      t.m[i] = make_map_nd(rows, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 3, dims, strides, box);
+    }
+  } else {
+    t.m[0] = make_map(rows, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, EM, (uint64_t)K * 2, 64, 16);
+    t.m[1] = make_map(rows, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, EM, (uint64_t)K * 2, 64, 64);
+  }
+  return t;
 }
 
 int max_tok_tiles(int EM) { return EM / 16 + 1; }
@@ -1124,7 +1144,7 @@ bool pair_fits(const GemmParams& p, bool gateup) {
 }
 
 template <bool GATEUP, int KS, int CTAS>
-void launch_gemm_ks(const CUtensorMap& tw, const CUtensorMap& tb, const CUtensorMap& tb64, GemmParams p,
+void launch_gemm_ks(const CUtensorMap& tw, const TokMaps& tb, GemmParams p,
                     cudaStream_t stream) {
   // Shared memory: token stages (this CTA's rows x KS), scales (double-buffered when they fit),
   // barriers, epilogue staging; what is left becomes the packed-weight ring (3..8 stages of
@@ -1169,7 +1189,7 @@ void launch_gemm_ks(const CUtensorMap& tw, const CUtensorMap& tb, const CUtensor
     if (dev >= 0 && dev < 64) configured[dev].store(true);
   }
   if (CTAS == 1) {
-    moe_gemm_sm100_kernel<GATEUP, KS, CTAS><<<sm_count(), kThreads, smem, stream>>>(tw, tb, tb64, p);
+    moe_gemm_sm100_kernel<GATEUP, KS, CTAS><<<sm_count(), kThreads, smem, stream>>>(tw, tb, p);
   } else {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(sm_count() & ~1));
@@ -1183,18 +1203,18 @@ void launch_gemm_ks(const CUtensorMap& tw, const CUtensorMap& tb, const CUtensor
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    VK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, moe_gemm_sm100_kernel<GATEUP, KS, CTAS>, tw, tb, tb64, p));
+    VK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, moe_gemm_sm100_kernel<GATEUP, KS, CTAS>, tw, tb, p));
   }
 }
 
 // Stage length and CTA grouping by the largest token tile of the launch (see the kernel's comment).
 template <bool GATEUP>
-void launch_gemm(const CUtensorMap& tw, const CUtensorMap& tb, const CUtensorMap& tb64, GemmParams p,
+void launch_gemm(const CUtensorMap& tw, const TokMaps& tb, GemmParams p,
                  bool use_pair, cudaStream_t stream) {
-  if (p.max_tok <= 64) launch_gemm_ks<GATEUP, 256, 1>(tw, tb, tb64, p, stream);
-  else if (p.max_tok <= 128) launch_gemm_ks<GATEUP, 128, 1>(tw, tb, tb64, p, stream);
-  else if (use_pair) launch_gemm_ks<GATEUP, 128, 2>(tw, tb, tb64, p, stream);
-  else launch_gemm_ks<GATEUP, 64, 1>(tw, tb, tb64, p, stream);
+  if (p.max_tok <= 64) launch_gemm_ks<GATEUP, 256, 1>(tw, tb, p, stream);
+  else if (p.max_tok <= 128) launch_gemm_ks<GATEUP, 128, 1>(tw, tb, p, stream);
+  else if (use_pair) launch_gemm_ks<GATEUP, 128, 2>(tw, tb, p, stream);
+  else launch_gemm_ks<GATEUP, 64, 1>(tw, tb, p, stream);
 }
 
 }  // namespace
@@ -1475,21 +1495,14 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
   g.sorted_ids = sorted_ids; g.tiles = tiles; g.n_tiles = n_tiles;
   g.N = M * top_k; g.top_k = top_k; g.w_sorted = w_sorted; g.activation = activation;
   g.limit = swiglu_limit; g.beta = beta; g.linear_beta = linear_beta; g.max_tok = max_tok;
-  // token operand: bf16 rows [EM, K]
-  auto token_maps = [&](const void* rows, int K, CUtensorMap& tb, CUtensorMap& tb64) {
-    tb = make_map(rows, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, EM, (uint64_t)K * 2, 64, 16);
-    tb64 = make_map(rows, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, EM, (uint64_t)K * 2, 64, 64);
-  };
-
   {  // gate/up
     GemmParams p = g;
     p.w_scale = w13_scale; p.bias = b13; p.act = act_scratch;
     p.K = hidden; p.n_feat = ispp; p.n_ftiles = ispp / 64;
     const CUtensorMap tw = make_map(w13, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, hidden / 2, w13_rows_cap, hidden / 2, 128, 64);
-    CUtensorMap tb, tb64;
-    token_maps(gathered, hidden, tb, tb64);
+    const TokMaps tb = token_maps(gathered, hidden, EM, use_pair);
     timer_mark(0, stream);
-    launch_gemm<true>(tw, tb, tb64, p, use_pair, stream);
+    launch_gemm<true>(tw, tb, p, use_pair, stream);
     timer_mark(1, stream);
   }
   {  // down + combine
@@ -1502,9 +1515,8 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
       p.raw_ld = hidden;
     }
     const CUtensorMap tw = make_map(w2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, ispp / 2, w13_rows_cap, ispp / 2, 128, 64);
-    CUtensorMap tb, tb64;
-    token_maps(act_scratch, ispp, tb, tb64);
-    launch_gemm<false>(tw, tb, tb64, p, use_pair, stream);
+    const TokMaps tb = token_maps(act_scratch, ispp, EM, use_pair);
+    launch_gemm<false>(tw, tb, p, use_pair, stream);
     timer_mark(2, stream);
   }
   if (ordered)
@@ -1556,18 +1568,15 @@ void launch_moe_stage_gemm(int which, const uint16_t* rows_in, const uint8_t* w,
   p.n_feat = n_out;
   const uint64_t rows_cap = (uint64_t)1 << 31;
   const CUtensorMap tw = make_map(w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, k_shard / 2, rows_cap, k_shard / 2, 128, 64);
-  const CUtensorMap tb = make_map(token_rows, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k_full, EM,
-                                  (uint64_t)k_full * 2, 64, 16);
-  const CUtensorMap tb64 = make_map(token_rows, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, k_full, EM,
-                                    (uint64_t)k_full * 2, 64, 64);
+  const TokMaps tb = token_maps(token_rows, k_full, EM, choice.use_pair);
   if (which == 0) {
     p.n_ftiles = n_out / 64;
     p.raw_ld = 2 * n_out;
-    launch_gemm<true>(tw, tb, tb64, p, choice.use_pair, stream);
+    launch_gemm<true>(tw, tb, p, choice.use_pair, stream);
   } else {
     p.n_ftiles = (n_out + 127) / 128;
     p.raw_ld = n_out;
-    launch_gemm<false>(tw, tb, tb64, p, choice.use_pair, stream);
+    launch_gemm<false>(tw, tb, p, choice.use_pair, stream);
   }
   VK_CUDA_CHECK(cudaGetLastError());
 }

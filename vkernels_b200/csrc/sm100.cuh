@@ -296,12 +296,11 @@ __device__ __forceinline__ void mbar_arrive_cta(uint32_t bar, uint32_t cta) {
 // Token-tile load of a CTA pair: the data lands in THIS CTA's shared memory, the
 // transaction bytes are credited to the barrier at the same offset in the pair's
 // leader (even) CTA, whose MMA thread consumes both halves. No multicast.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y,
-                                                 uint32_t bar) {
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(x), "r"(y), "r"(bar & 0xFEFFFFFFu)
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar & 0xFEFFFFFFu)
       : "memory");
 }
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
