@@ -618,6 +618,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         // Per 8 token columns the warp reads its two 16-lane groups in the 16x256b shape: a thread then holds gate and
         // up of (feature lane / 4 [+ 8], tokens 2 (lane % 4) and the next one).
         const bool situ = p.activation == 1;   // uniform across the launch
+        const float clamp = p.limit > 0.0f ? p.limit : INFINITY;
         const int fl = q * 16 + (lane >> 2);
         const int tk = (lane & 3) * 2;
         float bg[2] = {0.f, 0.f}, bu[2] = {0.f, 0.f};
@@ -627,7 +628,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
         uint16_t* const stage = reinterpret_cast<uint16_t*>(epi_smem) + es * (16 * kEpiPitch);
         for (int c0 = 0; c0 < n_tok; c0 += 8) {
-          float a[2][4];   // [lane group][gate, gate, up, up] of two tokens
+          float acc[2][4];   // [lane group][gate, gate, up, up] of two tokens
 #pragma unroll
           for (int d0 = 0; d0 < kDigits; d0 += 3) {   // three planes at a time, for the registers' sake
             float v[3][2][4];
@@ -640,7 +641,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             tc_wait_ld();
 #pragma unroll
             for (int i = 0; i < 8; ++i) {   // digit planes: 8^d each, the largest last
-              float& s = a[i >> 2][i & 3];
+              float& s = acc[i >> 2][i & 3];
               s = d0 == 0 ? v[0][i >> 2][i & 3] : s * 0.125f + v[0][i >> 2][i & 3];
               s = s * 0.125f + v[1][i >> 2][i & 3];
               s = s * 0.125f + v[2][i >> 2][i & 3];
@@ -651,19 +652,32 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           for (int e = 0; e < 2; ++e) {
             const int t = c0 + tk + e;
             const float ts = tile_s[t];
-            uint16_t* d = stage + t * kEpiPitch + fl;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              float g = a[h][e] * ts, u = a[h][2 + e] * ts;
-              if (bad && tile_ref[t] != 0ull) {
-                const size_t r = (size_t)wk.tt.expert * n_wrows + f * 64 + fl + 8 * h;
-                g += nonfinite(r, t);
-                u += nonfinite(r + p.n_feat, t);
-              }
-              g += bg[h];
-              u += bu[h];
-              d[8 * h] = f32_to_bf16_bits(situ ? moe_act_value(1, g, u, p.limit, p.beta, p.linear_beta) : swiglu_fast(g, u, p.limit));
+              acc[h][e] *= ts;
+              acc[h][2 + e] *= ts;
             }
+            if (bad && tile_ref[t] != 0ull) {
+              for (int h = 0; h < 2; ++h) {
+                const size_t r = (size_t)wk.tt.expert * n_wrows + f * 64 + fl + 8 * h;
+                acc[h][e] += nonfinite(r, t);
+                acc[h][2 + e] += nonfinite(r + p.n_feat, t);
+              }
+            }
+          }
+          uint16_t* const d = stage + (c0 + tk) * kEpiPitch + fl;
+          if (!situ) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                d[e * kEpiPitch + 8 * h] = f32_to_bf16_bits(swiglu_fast(acc[h][e] + bg[h], acc[h][2 + e] + bu[h], clamp));
+          } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                d[e * kEpiPitch + 8 * h] = f32_to_bf16_bits(moe_act_value(1, acc[h][e] + bg[h], acc[h][2 + e] + bu[h], p.limit, p.beta, p.linear_beta));
           }
         }
         // rows leave as 16-byte pieces: 8 consecutive threads write one 128-byte act row

@@ -90,10 +90,8 @@ constexpr int block_threads(int ctas) { return (4 + 4 * (dequant_sets(ctas) + ep
 constexpr int kPackedSfBytes = kRows * 8;   // prepacked scale factors of a 128-row, 256-K stage
 constexpr int kTmemCols = 512;
 constexpr int kEpiPitch = 72;                     // bf16 per staged token row: 64 features + 16 bytes against bank conflicts
-constexpr int kEpiStageBytes = 2 * 2 * 32 * kEpiPitch * 2;   // gate/up epilogue staging (two rounds per set, up to two sets)
-constexpr int kEpiStageDownBytes = 4 * 32 * 32 * 4;   // down epilogue: one 32 x 32 fp32 block per warp
-// what a launch really stages: a lone CTA runs one epilogue set, half of the above
-constexpr int epi_stage_bytes(bool gateup, int ctas) { return (gateup ? kEpiStageBytes : kEpiStageDownBytes) / (ctas == 2 ? 1 : 2); }
+// epilogue staging: gate/up two rounds of 32 tokens per set, down one 16 x 32 fp32 block per warp
+constexpr int epi_stage_bytes(bool gateup, int ctas) { return epi_sets(ctas) * (gateup ? 2 * 32 * kEpiPitch * 2 : 4 * 16 * 32 * 4); }
 // Lone-CTA form: byte -> bf16 pair lookup table in shared memory, one copy per bank (lane l reads
 // word 32 * byte + l), so a warp's 32 lookups of different bytes are one conflict-free access.
 constexpr int kLutBytes = 256 * 32 * 4;
@@ -654,6 +652,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
         // a thread then holds gate and up of (feature lane / 4 [+ 8], tokens 8i + 2 * (lane % 4)
         // and the next one), so the activation needs no exchange between lanes.
         const bool situ = p.activation == 1;   // uniform across the launch
+        const float clamp = p.limit > 0.0f ? p.limit : INFINITY;
         const int fl = q * 16 + (lane >> 2);   // feature inside the item's 64, first lane group
         const int tk = (lane & 3) * 2;
         float bg[2] = {0.f, 0.f}, bu[2] = {0.f, 0.f};
@@ -689,24 +688,36 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
           // a ballot, so the stores below depend on no load
           const int my_t = c0 + lane;
           const unsigned real = __ballot_sync(0xFFFFFFFFu, my_t < tt.n_rows && bars->tile_ref[my_t] != 0ull);
-          // activation -> bf16 into the staging tile [token][feature] of this round ...
+          // activation -> bf16 into the staging tile [token][feature] of this round ... (one straight line of sixteen
+          // independent elements: a warp alone on its scheduler's slot is bound by their latency)
           uint16_t* stg = my_stage + (round & 1) * (32 * kEpiPitch) + tk * kEpiPitch + fl;
+          uint16_t act[4][2][2];
+          if (!situ) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                act[i][e][0] = f32_to_bf16_bits(swiglu_fast(__uint_as_float(va[4 * i + e]) + bg[0], __uint_as_float(va[4 * i + 2 + e]) + bu[0], clamp));
+                act[i][e][1] = f32_to_bf16_bits(swiglu_fast(__uint_as_float(vb[4 * i + e]) + bg[1], __uint_as_float(vb[4 * i + 2 + e]) + bu[1], clamp));
+              }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                act[i][e][0] = f32_to_bf16_bits(moe_act_value(1, __uint_as_float(va[4 * i + e]) + bg[0], __uint_as_float(va[4 * i + 2 + e]) + bu[0],
+                                                              p.limit, p.beta, p.linear_beta));
+                act[i][e][1] = f32_to_bf16_bits(moe_act_value(1, __uint_as_float(vb[4 * i + e]) + bg[1], __uint_as_float(vb[4 * i + 2 + e]) + bu[1],
+                                                              p.limit, p.beta, p.linear_beta));
+              }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const float g0 = __uint_as_float(va[4 * i + e]) + bg[0], u0 = __uint_as_float(va[4 * i + 2 + e]) + bu[0];
-              const float g1 = __uint_as_float(vb[4 * i + e]) + bg[1], u1 = __uint_as_float(vb[4 * i + 2 + e]) + bu[1];
-              uint16_t* d = stg + (8 * i + e) * kEpiPitch;
-              if (!situ) {
-                d[0] = f32_to_bf16_bits(swiglu_fast(g0, u0, p.limit));
-                d[8] = f32_to_bf16_bits(swiglu_fast(g1, u1, p.limit));
-              } else {
-                d[0] = f32_to_bf16_bits(moe_act_value(1, g0, u0, p.limit, p.beta, p.linear_beta));
-                d[8] = f32_to_bf16_bits(moe_act_value(1, g1, u1, p.limit, p.beta, p.linear_beta));
-              }
+              stg[(8 * i + e) * kEpiPitch] = act[i][e][0];
+              stg[(8 * i + e) * kEpiPitch + 8] = act[i][e][1];
             }
-          }
           // ... then rows leave as 16-byte pieces: 8 consecutive threads write one 128-byte act row.
           // One barrier per round: a buffer is rewritten two rounds later, after the barrier of
           // the round in between, which every reader of this round has passed by then.
@@ -743,34 +754,45 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
             if (c0 + 32 * kEpiSets >= tt.n_rows) release_acc();   // this warp's last read of the accumulator
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
+              // this lane's four tokens of the half, looked up before the block turns around
+              unsigned long long ref[4];
+              float wgt[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int t = c0 + half * 16 + (lane >> 3) + 4 * i;
+                const bool in = t < tt.n_rows && quad_ok;
+                ref[i] = in ? (p.raw != nullptr ? 1ull : bars->tile_ref[t]) : 0ull;
+                wgt[i] = in ? bars->tile_w[t] : 0.0f;
+              }
               __syncwarp();   // the previous block has been read
 #pragma unroll
               for (int j = 0; j < 16; ++j) stage[j * 32 + lane] = __uint_as_float(v[half * 16 + j]);
               __syncwarp();
+              float4 a[4];
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
-                const int tl = (lane >> 3) + 4 * i;
-                const int t = c0 + half * 16 + tl;
-                if (p.raw != nullptr) {   // plain partial rows, no bias, no routing weight
-                  if (t < tt.n_rows && quad_ok) {
-                    float4 a = *reinterpret_cast<const float4*>(stage + tl * 32 + hq);
-                    *reinterpret_cast<float4*>(p.raw + (size_t)(tt.row0 + t) * p.raw_ld + h0) = a;
-                  }
-                  continue;
-                }
-                float* orow = t < tt.n_rows ? reinterpret_cast<float*>(bars->tile_ref[t]) : nullptr;
-                if (orow != nullptr && quad_ok) {
-                  const float wgt = bars->tile_w[t];
-                  float4 a = *reinterpret_cast<const float4*>(stage + tl * 32 + hq);
-                  if (p.store_rows)   // plain 16-byte store of the slot's row; the home rank adds its slots in order
-                    *reinterpret_cast<float4*>(orow + h0) = make_float4(a.x + b4.x, a.y + b4.y, a.z + b4.z, a.w + b4.w);
-                  else if (p.out_rows != nullptr)
-                    red_add_v4_sys(orow + h0, (a.x + b4.x) * wgt, (a.y + b4.y) * wgt,
-                                   (a.z + b4.z) * wgt, (a.w + b4.w) * wgt);
-                  else
-                    red_add_v4(orow + h0, (a.x + b4.x) * wgt, (a.y + b4.y) * wgt,
-                               (a.z + b4.z) * wgt, (a.w + b4.w) * wgt);
-                }
+                a[i] = *reinterpret_cast<const float4*>(stage + ((lane >> 3) + 4 * i) * 32 + hq);
+                a[i].x += b4.x; a[i].y += b4.y; a[i].z += b4.z; a[i].w += b4.w;   // (no bias with plain rows)
+              }
+              if (p.raw != nullptr) {   // plain partial rows, no bias, no routing weight
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (ref[i] != 0ull)
+                    *reinterpret_cast<float4*>(p.raw + (size_t)(tt.row0 + c0 + half * 16 + (lane >> 3) + 4 * i) * p.raw_ld + h0) = a[i];
+              } else if (p.store_rows) {   // plain 16-byte store of the slot's row; the home rank adds its slots in order
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (ref[i] != 0ull) *reinterpret_cast<float4*>(reinterpret_cast<float*>(ref[i]) + h0) = a[i];
+              } else if (p.out_rows != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (ref[i] != 0ull)
+                    red_add_v4_sys(reinterpret_cast<float*>(ref[i]) + h0, a[i].x * wgt[i], a[i].y * wgt[i], a[i].z * wgt[i], a[i].w * wgt[i]);
+              } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  if (ref[i] != 0ull)
+                    red_add_v4(reinterpret_cast<float*>(ref[i]) + h0, a[i].x * wgt[i], a[i].y * wgt[i], a[i].z * wgt[i], a[i].w * wgt[i]);
               }
             }
           }
@@ -843,36 +865,49 @@ build_tiles_kernel(const int32_t* __restrict__ expert_ids, int n_blocks, int blo
   build_tiles_block<1024>(expert_ids, n_blocks, block_size, max_tok, tiles, n_tiles, max_tiles, warp_sums);
 }
 
-// A_sorted[r, :] = A[sorted_ids[r] / top_k, :] (or the row at A_rows[sorted_ids[r] / top_k]) for
-// real rows, zeros otherwise: four rows per CTA, 256 threads each. The CTA after the last row
-// CTA builds the token-tile list instead (tiles != nullptr), so that the list costs no launch
-// of its own and is ready when the rows are.
-__global__ void __launch_bounds__(1024)
+// A_sorted[r, :] = A[sorted_ids[r] / top_k, :] (or the row at A_rows[sorted_ids[r] / top_k]) for real rows; padding rows
+// become zeros if `zero_pad` (the plain-result GEMM writes its results for them) and are left alone otherwise: a padding
+// column's results are never read. A warp per row with four 16-byte vectors a lane in flight: the copy is bound by the
+// bytes in flight (8192 tokens x 4 x 5760 bytes: 104 us with one vector a thread in flight, 256 threads a row). CTA 0
+// builds the token-tile list instead (tiles != nullptr), so that the list costs no launch of its own and is ready
+// when the rows are.
+constexpr int kGatherWarps = 8;
+__global__ void __launch_bounds__(32 * kGatherWarps)
 gather_rows_kernel(const uint16_t* __restrict__ A, const uint16_t* const* __restrict__ A_rows,
                    const int32_t* __restrict__ sorted_ids,
                    const int32_t* __restrict__ expert_ids, int block_size, int EM, int N, int top_k,
-                   int H, uint16_t* __restrict__ dst, int32_t* __restrict__ inv, int max_tok,
+                   int H, uint16_t* __restrict__ dst, int32_t* __restrict__ inv, int zero_pad, int max_tok,
                    TokTile* __restrict__ tiles, int* __restrict__ n_tiles, int max_tiles) {
-  if ((int)blockIdx.x * 4 >= EM) {   // the extra CTA
-    __shared__ int warp_sums[32];
+  if (blockIdx.x == 0) {
+    __shared__ int warp_sums[kGatherWarps];
     if (tiles != nullptr)
-      build_tiles_block<1024>(expert_ids, EM / block_size, block_size, max_tok, tiles, n_tiles, max_tiles, warp_sums);
+      build_tiles_block<32 * kGatherWarps>(expert_ids, EM / block_size, block_size, max_tok, tiles, n_tiles, max_tiles, warp_sums);
     return;
   }
-  const int vec_per_row = H / 8;  // 16-byte vectors
-  const int r = blockIdx.x * 4 + (threadIdx.x >> 8), t = threadIdx.x & 255;
+  const int lane = threadIdx.x & 31;
+  const int r = ((int)blockIdx.x - 1) * kGatherWarps + (threadIdx.x >> 5);
   if (r >= EM) return;
   if (expert_ids[r / block_size] < 0) return;  // never read by any tile
   const int flat = sorted_ids[r];
   const bool real = flat >= 0 && flat < N;
+  if (!real && zero_pad == 0) return;
   const int token = real ? flat / top_k : 0;
-  if (real && inv != nullptr && t == 0) inv[flat] = r;
+  if (real && inv != nullptr && lane == 0) inv[flat] = r;
   // a row address from A_rows may lie in another GPU's memory (peer load over NVLink)
   const uint4* src = reinterpret_cast<const uint4*>(
       A_rows != nullptr ? (real ? A_rows[token] : nullptr) : A + (size_t)token * H);
   uint4* d = reinterpret_cast<uint4*>(dst + (size_t)r * H);
-  for (int i = t; i < vec_per_row; i += 256)
-    d[i] = real ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+  const int n_vec = H / 8;  // 16-byte vectors
+  constexpr int kFlight = 4;
+  for (int i0 = lane; i0 < n_vec; i0 += 32 * kFlight) {
+    uint4 v[kFlight];
+#pragma unroll
+    for (int j = 0; j < kFlight; ++j)
+      v[j] = real && i0 + 32 * j < n_vec ? src[i0 + 32 * j] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int j = 0; j < kFlight; ++j)
+      if (i0 + 32 * j < n_vec) d[i0 + 32 * j] = v[j];
+  }
 }
 
 // Ordered combine: y[t, :] = bf16( sum over the token's routed slots, in ascending sorted-row
@@ -1138,7 +1173,7 @@ bool pair_mode() {
 // at least two packed-weight stages.
 bool pair_fits(const GemmParams& p, bool gateup) {
   const int scale_tile = (128 * (p.K / 32) + 127) & ~127;
-  const int fixed = 1024 + (((int)sizeof(Barriers) + 127) & ~127) + (gateup ? kEpiStageBytes : kEpiStageDownBytes) + 128;
+  const int fixed = 1024 + (((int)sizeof(Barriers) + 127) & ~127) + epi_stage_bytes(gateup, 2) + 128;
   const int tokens = 6 * (((p.max_tok + 31) >> 5) << 4) * 128;   // 6 x 64-K or 3 x 128-K slots
   return 227 * 1024 - fixed - scale_tile - tokens >= 2 * kWStageBytes;
 }
@@ -1487,9 +1522,9 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
     return;
   }
   // (a large one's by an extra CTA of the row gather)
-  gather_rows_kernel<<<(EM + 3) / 4 + 1, 1024, 0, stream>>>(A, a_rows, sorted_ids, expert_ids, block_size, EM, M * top_k,
-                                                           top_k, hidden, gathered, inv, max_tok, tiles, n_tiles,
-                                                           max_tok_tiles(EM));
+  gather_rows_kernel<<<(EM + kGatherWarps - 1) / kGatherWarps + 1, 32 * kGatherWarps, 0, stream>>>(
+      A, a_rows, sorted_ids, expert_ids, block_size, EM, M * top_k, top_k, hidden, gathered, inv, 0, max_tok, tiles, n_tiles,
+      max_tok_tiles(EM));
 
   GemmParams g{};
   g.sorted_ids = sorted_ids; g.tiles = tiles; g.n_tiles = n_tiles;
@@ -1557,8 +1592,9 @@ void launch_moe_stage_gemm(int which, const uint16_t* rows_in, const uint8_t* w,
                                              n_tiles, max_tok_tiles(EM));
   const uint16_t* token_rows = rows_in;
   if (which == 0) {
-    gather_rows_kernel<<<(EM + 3) / 4, 1024, 0, stream>>>(rows_in, nullptr, sorted_ids, expert_ids, block_size, EM,
-                                                          M * top_k, top_k, k_full, gathered, nullptr, 0, nullptr, nullptr, 0);
+    gather_rows_kernel<<<(EM + kGatherWarps - 1) / kGatherWarps + 1, 32 * kGatherWarps, 0, stream>>>(
+        rows_in, nullptr, sorted_ids, expert_ids, block_size, EM, M * top_k, top_k, k_full, gathered, nullptr, 1, 0, nullptr,
+        nullptr, 0);
     token_rows = gathered;
   }
   GemmParams p{};

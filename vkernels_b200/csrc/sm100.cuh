@@ -217,13 +217,6 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(pred));
   return pred != 0;
 }
-// SwiGLU with the hardware exp / reciprocal approximations (relative error
-// ~1e-6, far inside the layer's tolerance; the CUDA-core cross-check path keeps
-// the accurate functions). Straight-line code - no data-dependent branch - so
-// the 16 elements a thread finishes per round overlap their latencies. inf and
-// NaN come out as in the CPU definition: NaN stays NaN (comparisons with NaN
-// are false), +inf gives inf * u, and -inf, where the definition evaluates
-// -inf / inf = NaN, is patched by the final select.
 __device__ __forceinline__ float fmin_nan(float a, float b) {   // NaN if either operand is NaN
   float r;
   asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
@@ -234,15 +227,20 @@ __device__ __forceinline__ float fmax_nan(float a, float b) {
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
-__device__ __forceinline__ float swiglu_fast(float g, float u, float limit) {
-  if (limit > 0.0f) {   // uniform across the launch; a NaN operand stays NaN
-    g = fmin_nan(g, limit);
-    u = fmax_nan(fmin_nan(u, limit), -limit);
-  }
-  // exp(-g) overflows fp32 beyond 88; the quotient is below 1e-36 in magnitude either way.
-  const float ng = fminf(-g, 87.0f);
-  const float r = __fdividef(g, 1.0f + __expf(ng));
-  return ((g == -INFINITY) ? __int_as_float(0x7FC00000) : r) * u;
+// SwiGLU, g / (1 + exp(-g)) * u, with the hardware's exp2 and reciprocal approximations (relative error ~1e-6, far
+// inside the layer's tolerance; the CUDA-core cross-check path keeps the accurate functions). The prefill epilogues are
+// bound by these instructions - two on the special-function unit and the rest on half-rate pipes, 16 elements a thread
+// and round - so there is nothing here but them: flushed subnormals (exp of a large positive g next to 1, the
+// quotient of a g below -87), no branch, no range fix. inf and NaN come out as in the CPU definition without one:
+// NaN stays NaN; +inf gives inf * u; for -inf the sum is inf, its reciprocal 0, and -inf * 0 = NaN, as -inf / inf is there.
+// `clamp` is the limit, or +inf for none (the clamps then change nothing, NaN included).
+__device__ __forceinline__ float swiglu_fast(float g, float u, float clamp) {
+  g = fmin_nan(g, clamp);
+  u = fmax_nan(fmin_nan(u, clamp), -clamp);
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return g * r * u;
 }
 // ---- CTA-pair (cta_group::2) helpers ---------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
