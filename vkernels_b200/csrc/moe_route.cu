@@ -649,9 +649,9 @@ void router_logits(const uint16_t* x, const float* wr, float* logits, int T, int
   const bool aligned16 = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(wr) & 15u) == 0;
   const bool tc = router_tc_mode() && H % 64 == 0 && E % 16 == 0 && E <= 256 && aligned16;
   // Up to 512 tokens the dot-product kernels read the weight row again for every token. That is cheaper than the tensor-core
-  // kernel's three launches (about 12 us) up to some 16 million products: 8 us at 128 x 32 x 2880, but 21 us at 32 x 256
-  // x 7168 and 53 us at 333 x 128 x 2880.
-  if (tc && T <= 512 && (long long)T * E * H > (16ll << 20) &&
+  // kernel's three launches (15 us at 333 x 128 x 2880, where they take 53) up to some 32 million products (8 us at 128 x
+  // 32 x 2880), and up to 64 tokens in any case: there the weight's own split costs as much (21 us both at 32 x 256 x 7168).
+  if (tc && T > 64 && T <= 512 && (long long)T * E * H > (32ll << 20) &&
       launch_router_tc(x, wr, logits, T, H, E, static_cast<cudaStream_t>(stream))) {
   } else if ((long long)T * E <= 8192 && T <= 65535 && H % 8 == 0 && aligned16) {
     router_logits_cta_kernel<<<dim3((unsigned)E, (unsigned)T), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, wr, logits, H, E);
