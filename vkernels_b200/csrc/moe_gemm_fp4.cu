@@ -25,9 +25,10 @@
 //
 // Warp roles (one persistent CTA per SM; every CTA takes a contiguous range of the (token tile,
 // feature tile) items, so that the tile's rows and scales are looked up once for many items):
-//   warp 0      TMA producer: packed weights (128 rows x 256 K a stage) and scale bytes
+//   warp 0      TMA producer: packed weights (128 rows x 256 K a stage)
 //   warp 1      tcgen05.mma issuer + tensor-memory allocation
 //   warp 2      TMA producer: digit planes of the token tile
+//   warp 3      checkpoint layout: the items' scale bytes (bulk copies)
 //   warps 4..   checkpoint layout: three teams of four warps (one per tensor-memory lane quarter),
 //               a stage each in turn: shared memory -> code rewrite -> tensor memory, scale factors
 //               prepacked weights: one team that only copies scale factors, the MMA reads the codes
@@ -67,7 +68,7 @@ constexpr int kSfBytes = kRows * 8;      // prepacked scale factors of a stage
 constexpr int kUnitCols = 16 * kDigits;  // accumulator columns of up to 16 tokens
 constexpr int kSfbCol = 2 * kUnitCols;
 constexpr int kSlot0 = kSfbCol + 8;
-constexpr int kMaxW = 8, kMaxSc = 8;
+constexpr int kMaxW = 8, kMaxSc = 8;   // weight slots (prepacked: all eight), scale buffers
 constexpr int kBadRing = 16;
 constexpr int kEpiSets = 2;
 constexpr int kEpiPitch = 72;            // bf16 per staged token row: 64 features + 16 bytes against bank conflicts
@@ -260,9 +261,9 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   Walk wk(p.tiles, *p.n_tiles, p.n_ftiles);
 
   if (warp == 0) {
-    // ------------------- TMA producer: packed weights + scales ---------------
+    // ------------------- TMA producer: packed weights -----------------------
     if (lane == 0) {
-      Ring w, sc, a;
+      Ring w, a;
       bool ok = true;
       for (; wk.left > 0 && ok; wk.next()) {
         if (PACKED) {
@@ -284,16 +285,6 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           const int row_a = GATEUP ? wk.tt.expert * n_wrows + wk.f * 64 : wk.tt.expert * n_wrows + wk.f * 128;
           const int row_b = GATEUP ? row_a + p.n_feat : row_a + 64;
           const bool both = GATEUP || p.n_feat - wk.f * 128 > 64;
-          {
-            if (!mbar_wait(smem_u32(&bars->sc_empty[sc.slot]), sc.phase ^ 1u, abort_flag, 1)) break;
-            const uint32_t bar = smem_u32(&bars->sc_full[sc.slot]);
-            const uint32_t dst = smem_u32(sc_smem + sc.slot * p.scale_buf_bytes);
-            const uint32_t half = 64u * pitch;
-            mbar_expect_tx(bar, both ? 2 * half : half);
-            bulk_load_1d(dst, p.w_scale + (size_t)row_a * pitch, half, bar);
-            if (both) bulk_load_1d(dst + half, p.w_scale + (size_t)row_b * pitch, half, bar);
-            sc.advance(p.scale_bufs);
-          }
           for (int kw = 0; kw < n_kw; ++kw) {
             if (!mbar_wait(smem_u32(&bars->w_empty[w.slot]), w.phase ^ 1u, abort_flag, 2)) {
               ok = false;
@@ -307,6 +298,25 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             w.advance(p.w_stages);
           }
         }
+      }
+    }
+  } else if (!PACKED && warp == 3) {
+    // ------------------- scale bytes, an item at a time ----------------------
+    // (a thread of its own: with one buffer, long K, the weights of the next item do not wait for it)
+    if (lane == 0) {
+      Ring sc;
+      for (; wk.left > 0; wk.next()) {
+        const int row_a = GATEUP ? wk.tt.expert * n_wrows + wk.f * 64 : wk.tt.expert * n_wrows + wk.f * 128;
+        const int row_b = GATEUP ? row_a + p.n_feat : row_a + 64;
+        const bool both = GATEUP || p.n_feat - wk.f * 128 > 64;
+        if (!mbar_wait(smem_u32(&bars->sc_empty[sc.slot]), sc.phase ^ 1u, abort_flag, 1)) break;
+        const uint32_t bar = smem_u32(&bars->sc_full[sc.slot]);
+        const uint32_t dst = smem_u32(sc_smem + sc.slot * p.scale_buf_bytes);
+        const uint32_t half = 64u * pitch;
+        mbar_expect_tx(bar, both ? 2 * half : half);
+        bulk_load_1d(dst, p.w_scale + (size_t)row_a * pitch, half, bar);
+        if (both) bulk_load_1d(dst + half, p.w_scale + (size_t)row_b * pitch, half, bar);
+        sc.advance(p.scale_bufs);
       }
     }
   } else if (warp == 2) {
@@ -458,6 +468,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         load_next();
         if (pf_lane) prefetch_stage();
         if (!mbar_wait(smem_u32(&bars->stage_done[sa.slot]), sa.phase ^ 1u, abort_flag, 9)) break;
+        __syncwarp();
         tc_fence_after();
         tc_st8(t_row + sa.slot * kACols, sf);
         tc_wait_st();
@@ -468,7 +479,10 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       }
     } else {
       // A team takes every kTeams-th stage of the CTA's running stage sequence: its ring positions advance by
-      // kTeams, and a weight slot is released by its team alone.
+      // kTeams, and a weight slot is released by its team alone. The weight ring's depth is a multiple of kTeams, so that
+      // a slot always belongs to one team: a barrier's parity tells a phase from the next one only to a waiter that has seen
+      // the phase before, and copies complete out of order - the team of stage i cannot conclude from its own stages that
+      // another team's load into the slot of i has landed.
       const int srow = GATEUP ? (((row >> 3) & 1) * 64 + (row >> 4) * 8 + (row & 7)) : row;   // row inside the staged tile
       int sf_row[4];
 #pragma unroll
@@ -476,9 +490,12 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const int L = 32 * i + lane;
         sf_row[i] = GATEUP ? (((L >> 3) & 1) * 64 + (L >> 4) * 8 + (L & 7)) : L;
       }
-      int w_slot = team % p.w_stages, a_slot = team;
-      uint32_t w_phase = (uint32_t)(team / p.w_stages) & 1u, a_phase = 0;
+      int w_slot = team, a_slot = team;
+      uint32_t w_phase = 0, a_phase = 0;
       int kw = team, seq = 0;   // stage inside the item; running number of the item
+      // A poll of a barrier costs over a hundred clocks even when its phase is complete, and these warps are bound by their
+      // latency: the coming stage's codes and this stage's slot are polled ahead of the work that hides it.
+      bool codes_seen = false;
       Ring sc;
       bool ok = true;
       for (; wk.left > 0 && ok; wk.next(), ++seq) {
@@ -486,10 +503,11 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (!mbar_wait(smem_u32(&bars->sc_full[sc.slot]), sc.phase, abort_flag, 7)) break;
         const uint8_t* sc_tile = sc_smem + sc.slot * p.scale_buf_bytes;
         for (; kw < n_kw; kw += kTeams) {
-          if (!mbar_wait(smem_u32(&bars->w_full[w_slot]), w_phase, abort_flag, 8)) {
+          if (!codes_seen && !mbar_wait(smem_u32(&bars->w_full[w_slot]), w_phase, abort_flag, 8)) {
             ok = false;
             break;
           }
+          const bool slot_seen = mbar_test(smem_u32(&bars->stage_done[a_slot]), a_phase ^ 1u);
           const uint8_t* my_row = w_smem + w_slot * kWBytes + srow * 128;
           uint32_t v[32];
 #pragma unroll
@@ -528,20 +546,22 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 #pragma unroll
             for (int i = 0; i < 8; ++i) sf[i] ^= ((sf[i] & 0x7F7F7F7Fu) + 0x01010101u) & sf[i] & 0x80808080u;   // 0xFF -> 0x7F
           }
-          if (!mbar_wait(smem_u32(&bars->stage_done[a_slot]), a_phase ^ 1u, abort_flag, 9)) {
+          if (!slot_seen && !mbar_wait(smem_u32(&bars->stage_done[a_slot]), a_phase ^ 1u, abort_flag, 9)) {
             ok = false;
             break;
           }
+          __syncwarp();   // the tensor-memory stores are warp-aligned; the lanes may have left the wait one by one
           tc_fence_after();
           const uint32_t slot_col = t_row + a_slot * kACols;
           tc_st32(slot_col, v);
           tc_st8(slot_col + kSfCol, sf);
+          w_slot += kTeams;
+          if (w_slot >= p.w_stages) { w_slot -= p.w_stages; w_phase ^= 1u; }
+          codes_seen = mbar_test(smem_u32(&bars->w_full[w_slot]), w_phase);
           tc_wait_st();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&bars->ready[a_slot]));
-          w_slot += kTeams;
-          while (w_slot >= p.w_stages) { w_slot -= p.w_stages; w_phase ^= 1u; }
           a_slot += kTeams;
           if (a_slot >= kASlots) { a_slot -= kASlots; a_phase ^= 1u; }
         }
@@ -596,6 +616,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
       const bool gave_up = !mbar_wait(smem_u32(&bars->acc_full[es]), phase, abort_flag, 10);
       phase ^= 1u;
       if (named_bar_or(bar_a, 128, gave_up)) break;
+      __syncwarp();
       tc_fence_after();
       const bool bad = !PACKED && *reinterpret_cast<volatile int*>(&bars->bad_item[seq % kBadRing]) == seq + 1;
       auto release_acc = [&]() {
@@ -796,7 +817,7 @@ __device__ __forceinline__ void digits8(const int (&v)[8], uint32_t (&out)[kDigi
 // are never read back. The gather variant also does two small jobs of the layer's front end: CTA 0
 // builds the token-tile list (tiles != nullptr), and every real row records where its routed slot
 // went (inv[flat] = r, when inv != nullptr).
-constexpr int kSplitThreads = 128;
+constexpr int kSplitThreads = 256;   // (128: the tile list of 240 tiles 4 us longer)
 constexpr int kHeld = 4;
 template <bool GATHER>
 __global__ void __launch_bounds__(kSplitThreads)
@@ -881,18 +902,24 @@ void launch_one(const CUtensorMap& tw, const CUtensorMap& tx8, const CUtensorMap
   const int fixed = 1024 + (((int)sizeof(Bars) + 127) & ~127) + kEpiBytes + 128;
   p.b_stage_bytes = (max_tok <= 8 ? 8 : (max_tok <= 16 ? 16 : 32)) * kDigits * 128;
   p.scale_buf_bytes = PACKED ? 0 : (kRows * (p.K / 32) + 16 + 127) & ~127;
-  // Enough scale buffers that short items do not hold the weight ring back (a buffer lasts an item), four token slots
-  // of the largest tiles or five of the small ones (they come from L2 with its full latency), and weight slots with what
-  // is left, at most eight: six (96 KB an SM) are what HBM takes to run at its rate.
-  const int n_kw = (p.K + kStageK - 1) / kStageK;
+  // Enough scale buffers that short items do not hold the code warps back (a buffer lasts an item), four token slots of the
+  // largest tiles or five of the small ones (they come from L2 with its full latency), six weight slots (96 KB an SM are what
+  // HBM takes to run at its rate; three where K is so long that its scale bytes fill the rest), and what is left for tokens
+  // again. The checkpoint layout wants a multiple of the teams (see the code warps).
+  const int n_kw = (p.K + kStageK - 1) / kStageK, want_w = PACKED ? kMaxW : 2 * teams(PACKED);
   p.scale_bufs = PACKED ? 0 : std::min(kMaxSc, 2 + (kMaxW - 1) / n_kw);
   p.b_stages = std::min(a_slots(PACKED), max_tok <= 8 ? 7 : (max_tok <= 16 || PACKED ? 5 : 4));
   auto room = [&]() { return (max_smem - fixed - p.scale_bufs * p.scale_buf_bytes - p.b_stages * p.b_stage_bytes) / kWBytes; };
+  while (room() < 6 && p.scale_bufs > 2) --p.scale_bufs;
   while (room() < 6 && p.b_stages > 4) --p.b_stages;
-  while (room() < 4 && p.scale_bufs > 1) --p.scale_bufs;
-  while (room() < 4 && p.b_stages > 2) --p.b_stages;
-  expects(room() >= 2, "fused_moe_mxfp4: reduction dimension too large for shared memory");
-  p.w_stages = std::min(kMaxW, room());
+  while (room() < 6 && p.scale_bufs > 1) --p.scale_bufs;
+  while (room() < 6 && p.b_stages > 3) --p.b_stages;
+  while (room() < 3 && p.b_stages > 1) --p.b_stages;
+  expects(room() >= 3, "fused_moe_mxfp4: reduction dimension too large for shared memory");
+  p.w_stages = std::min(room(), want_w);
+  if (!PACKED) p.w_stages -= p.w_stages % teams(PACKED);
+  while (p.b_stages < a_slots(PACKED) && (max_smem - fixed - p.scale_bufs * p.scale_buf_bytes - (p.b_stages + 1) * p.b_stage_bytes) / kWBytes >= p.w_stages)
+    ++p.b_stages;
   const int smem = fixed + p.scale_bufs * p.scale_buf_bytes + p.b_stages * p.b_stage_bytes + p.w_stages * kWBytes;
   static std::atomic<bool> configured[64];   // the attribute belongs to the device's context
   int dev = 0;
@@ -915,6 +942,7 @@ void launch_gemm_fp4(bool gateup, bool packed, Fp4Params p, const uint8_t* plane
   const CUtensorMap tx16 = sm100_make_map_u8(planes, 3, xdims, xstr, box16);
   CUtensorMap tw;
   if (packed) {
+    expects((reinterpret_cast<uintptr_t>(p.w) & 31u) == 0, "prepacked weights: 32-byte alignment, K a multiple of 64");
     // Accumulator row 16 g + 8 u + j: gate/up j = feature inside a group of 8, u = gate / up half, g = group; down: plain order.
     const uint64_t n_feat = (uint64_t)p.n_feat;
     const uint64_t dims[4] = {half, 8, 2, 1ull << 27};

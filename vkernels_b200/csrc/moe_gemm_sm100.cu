@@ -1441,10 +1441,10 @@ TileChoice choose_tiles(int M, int top_k, int EM, int block_size, int k_gateup, 
 }  // namespace
 
 // moe_gemm_fp4.cu takes tiles of up to 32 tokens. Where an expert sees eight on average or fewer, tiles end at 16 (a few
-// experts in a thousand hold more): the token slots are sized for the largest tile, and what they do not take holds weights.
-static int fp4_tile_limit(int M, int top_k, int EM, int block_size) {
-  if (M <= 8) return 16;
-  return M <= 16 || (long long)M * top_k <= 8 * experts_estimate(M, top_k, EM, block_size) ? 16 : 32;
+// experts in a thousand hold more): the token slots are sized for the largest tile, and what they do not take holds weights -
+// or, with a very long reduction, its scale bytes.
+static int fp4_tile_limit(int M, int top_k, int EM, int block_size, int max_k) {
+  return M <= 16 || max_k > 32768 || (long long)M * top_k <= 8 * experts_estimate(M, top_k, EM, block_size) ? 16 : 32;
 }
 
 // moe_gemv.cu
@@ -1496,7 +1496,7 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
   const uint64_t w13_rows_cap = (uint64_t)1 << 31;
   const TileChoice choice = choose_tiles(M, top_k, EM, block_size, hidden, ispp);
   const bool mx = choice.max_tok <= 64 && (small_fp4_mode() || w4);
-  const int max_tok = mx ? fp4_tile_limit(M, top_k, EM, block_size) : choice.max_tok;
+  const int max_tok = mx ? fp4_tile_limit(M, top_k, EM, block_size, std::max(hidden, ispp)) : choice.max_tok;
   expects(!w4 || mx, "fused_moe_mxfp4: prepacked weights serve decode-size batches only (token tiles of up to 64 rows); "
                      "larger batches take the checkpoint-layout weights");
   const bool use_pair = choice.use_pair;
