@@ -52,19 +52,18 @@ __device__ __forceinline__ uint32_t word_of(const uint4& v, int i) { return i ==
 // takes the 32-element group at 128 c + 32 q of every 128-K step c; column 0 of B is the
 // vector (threads with g == 0 carry it, read from shared memory), the other seven columns are
 // zero. Returns the two sums of column 0 in the threads with q == 0 (c[0]: row_lo, c[2]: row_hi).
-// The loads of the next kDepth steps are issued before the current ones are used: with ten
-// warps to an SM it is the bytes in flight per warp that decide how close to the memory rate
-// the kernel runs.
-constexpr int kDepth = 3;
+// The loads of the next DEPTH steps are issued before the current ones are used.
+template <int DEPTH>
 struct RowsBuf {
-  uint4 a[kDepth], b[kDepth];
-  uint32_t sa[kDepth], sb[kDepth];
+  uint4 a[DEPTH], b[DEPTH];
+  uint32_t sa[DEPTH], sb[DEPTH];
 };
-__device__ __forceinline__ void rows16_load(RowsBuf& r, const uint8_t* __restrict__ w_lo, const uint8_t* __restrict__ w_hi,
+template <int DEPTH>
+__device__ __forceinline__ void rows16_load(RowsBuf<DEPTH>& r, const uint8_t* __restrict__ w_lo, const uint8_t* __restrict__ w_hi,
                                             const uint8_t* __restrict__ s_lo, const uint8_t* __restrict__ s_hi, int k0,
                                             int k_end, int q) {
 #pragma unroll
-  for (int d = 0; d < kDepth; ++d) {
+  for (int d = 0; d < DEPTH; ++d) {
     const int k = k0 + 128 * d + 32 * q;
     r.a[d] = r.b[d] = make_uint4(0u, 0u, 0u, 0u);
     r.sa[d] = r.sb[d] = 0x7Fu;
@@ -76,10 +75,11 @@ __device__ __forceinline__ void rows16_load(RowsBuf& r, const uint8_t* __restric
     }
   }
 }
-__device__ __forceinline__ void rows16_use(const RowsBuf& r, const uint16_t* vec_smem, int k0, int k_end, int q, bool carries,
+template <int DEPTH>
+__device__ __forceinline__ void rows16_use(const RowsBuf<DEPTH>& r, const uint16_t* vec_smem, int k0, int k_end, int q, bool carries,
                                            float (&c)[4]) {
 #pragma unroll
-  for (int d = 0; d < kDepth; ++d) {
+  for (int d = 0; d < DEPTH; ++d) {
     const int k = k0 + 128 * d + 32 * q;
     uint4 x[4];
 #pragma unroll
@@ -99,13 +99,14 @@ __device__ __forceinline__ void rows16_use(const RowsBuf& r, const uint16_t* vec
     }
   }
 }
+template <int DEPTH>
 __device__ __forceinline__ void rows16_dot(const uint8_t* __restrict__ w_lo, const uint8_t* __restrict__ w_hi,
                                            const uint8_t* __restrict__ s_lo, const uint8_t* __restrict__ s_hi,
                                            const uint16_t* vec_smem, int k_begin, int k_end, int lane, float (&c)[4]) {
   const int q = lane & 3;
   const bool carries = (lane >> 2) == 0;
-  constexpr int kGroup = 128 * kDepth;
-  RowsBuf r0, r1;
+  constexpr int kGroup = 128 * DEPTH;
+  RowsBuf<DEPTH> r0, r1;
   int k0 = k_begin;
   if (k0 >= k_end) return;
   rows16_load(r0, w_lo, w_hi, s_lo, s_hi, k0, k_end, q);
@@ -142,23 +143,22 @@ __device__ __forceinline__ void k_piece(int K, int parts, int p, int& k_begin, i
   k_end = (p + 1) * len < K ? (p + 1) * len : K;
 }
 
-// grid (ispp / 32, N); 128 * kGateupParts threads = 4 feature warps (8 features each) x parts of
-// K whose sums meet in shared memory and are added in part order. Measured at one token of the
-// gpt-oss shapes: one part (four CTAs of four warps to an SM, all 360 CTAs resident at once) 21 us,
-// four parts (one CTA of sixteen warps to an SM by registers, three waves) 26 us - the kernel
-// is bound by instruction issue (integer pipe 51 % busy, 1.7 instructions per cycle), not by
-// the number of loads in flight.
-constexpr int kGateupParts = 1;
-__global__ void __launch_bounds__(128 * kGateupParts)
+// grid (ispp / 16, N); 128 threads = 2 feature warps (8 features each) x 2 parts of K whose sums meet in shared memory and are
+// added in part order. A warp is bound by the latency of its own chain - some 25 instructions per eight weights of
+// each of its rows - so the kernel wants as many warps as the registers hold at once: at one token of the gpt-oss shapes 720 CTAs, five to
+// an SM, 20.0 us, against 360 CTAs of four whole-K warps with three steps in flight, 22 us (four parts in one CTA of
+// sixteen warps, three waves: 26).
+constexpr int kGateupParts = 2, kGateupWarps = 4, kGateupFeat = 8 * (kGateupWarps / kGateupParts), kGateupDepth = 2;
+__global__ void __launch_bounds__(32 * kGateupWarps, 5)
 gemv_gateup_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ w13, const uint8_t* __restrict__ w13_scale,
                    const float* __restrict__ b13, const int32_t* __restrict__ sorted_ids,
                    const int32_t* __restrict__ expert_ids, int EM, int block_size, int top_k, int hidden, int ispp,
                    int activation, float limit, float beta, float linear_beta, uint16_t* __restrict__ act,
                    int32_t* __restrict__ slot_expert) {
   __shared__ int s_found;
-  __shared__ float part[4][kGateupParts][16];              // [feature warp][part][8 gate sums, 8 up sums]
+  __shared__ float part[kGateupWarps / kGateupParts][kGateupParts][16];   // [feature warp][part][8 gate sums, 8 up sums]
   extern __shared__ __align__(16) uint16_t vec_smem[];   // the token's row [hidden]
-  constexpr int kThreads = 128 * kGateupParts;
+  constexpr int kThreads = 32 * kGateupWarps;
   const int s = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int fw = warp / kGateupParts, pt = warp % kGateupParts;
   {
@@ -168,7 +168,7 @@ gemv_gateup_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ w
   const int e = find_slot_expert(sorted_ids, expert_ids, EM, block_size, s, tid, kThreads, &s_found);   // (its barriers publish the row)
   if (blockIdx.x == 0 && tid == 0) slot_expert[s] = e;
   if (e < 0) return;
-  const int f_warp = blockIdx.x * 32 + fw * 8;   // ispp is a multiple of 8: a warp's features are all in or all out
+  const int f_warp = blockIdx.x * kGateupFeat + fw * 8;   // ispp is a multiple of 8: a warp's features are all in or all out
   if (f_warp < ispp) {
     const int g = lane >> 2;
     const size_t row_g = (size_t)e * 2 * ispp + f_warp + g, row_u = row_g + ispp;
@@ -176,7 +176,7 @@ gemv_gateup_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ w
     int k_begin, k_end;
     k_piece(hidden, kGateupParts, pt, k_begin, k_end);
     float c[4] = {0.f, 0.f, 0.f, 0.f};
-    rows16_dot(w13 + row_g * pitch, w13 + row_u * pitch, w13_scale + row_g * spitch, w13_scale + row_u * spitch, vec_smem,
+    rows16_dot<kGateupDepth>(w13 + row_g * pitch, w13 + row_u * pitch, w13_scale + row_g * spitch, w13_scale + row_u * spitch, vec_smem,
                k_begin, k_end, lane, c);
     if ((lane & 3) == 0) {
       part[fw][pt][g] = c[0];
@@ -184,8 +184,8 @@ gemv_gateup_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ w
     }
   }
   __syncthreads();
-  if (tid < 32) {
-    const int w = tid >> 3, g = tid & 7, f = blockIdx.x * 32 + w * 8 + g;
+  if (tid < kGateupFeat) {
+    const int w = tid >> 3, g = tid & 7, f = blockIdx.x * kGateupFeat + w * 8 + g;
     if (f < ispp) {
       float gs = 0.0f, us = 0.0f;
 #pragma unroll
@@ -203,7 +203,9 @@ gemv_gateup_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ w
 }
 
 // grid (hidden / 16, M); 32 * KSPLIT * top_k threads (at most 512): warp KSPLIT * j + h = slot j of
-// the token, part h of K (two halves while top_k <= 8, else the whole of it).
+// the token, part h of K (two halves while top_k <= 8, else the whole of it). Quarters with one step in flight, so that
+// two CTAs share an SM, are no faster (15.9 us for 15.5 at one token, hidden = ispp = 2880).
+constexpr int kDownDepth = 3;
 template <int KSPLIT>
 __global__ void __launch_bounds__(512)
 gemv_down_kernel(const uint16_t* __restrict__ act, const uint8_t* __restrict__ w2, const uint8_t* __restrict__ w2_scale,
@@ -233,7 +235,7 @@ gemv_down_kernel(const uint16_t* __restrict__ act, const uint8_t* __restrict__ w
     int k_begin, k_end;
     k_piece(ispp, KSPLIT, half, k_begin, k_end);
     float c[4] = {0.f, 0.f, 0.f, 0.f};
-    rows16_dot(w2 + row_lo * pitch, w2 + row_hi * pitch, w2_scale + row_lo * spitch, w2_scale + row_hi * spitch,
+    rows16_dot<kDownDepth>(w2 + row_lo * pitch, w2 + row_hi * pitch, w2_scale + row_lo * spitch, w2_scale + row_hi * spitch,
                act_smem + (size_t)j * ispp, k_begin, k_end, lane, c);
     if ((lane & 3) == 0) {
       part[j][half][g] = c[0];
@@ -303,7 +305,7 @@ void launch_moe_tiny(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_s
       if (dev >= 0 && dev < 64) configured[dev].store(smem_down);
     }
   }
-  gemv_gateup_kernel<<<dim3((unsigned)((ispp + 31) / 32), (unsigned)N), 128 * kGateupParts, (size_t)hidden * sizeof(uint16_t), stream>>>(
+  gemv_gateup_kernel<<<dim3((unsigned)((ispp + kGateupFeat - 1) / kGateupFeat), (unsigned)N), 32 * kGateupWarps, (size_t)hidden * sizeof(uint16_t), stream>>>(
       A, w13, w13_scale, b13, sorted_ids, expert_ids, EM, block_size, top_k, hidden, ispp, activation, swiglu_limit, beta,
       linear_beta, act, slot_expert);
   const dim3 grid_down((unsigned)(hidden / 16), (unsigned)M);
