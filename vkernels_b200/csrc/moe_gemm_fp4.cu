@@ -19,9 +19,9 @@
 //
 // What bounds it: the weight bytes. Per 128 rows x 256 K (17 KB) an SM gets its share of HBM in about 700 clocks. A
 // stage takes about 720 prepacked and 950 to 1000 from the checkpoint layout (the code warps' latency); with one byte a
-// weight it took 1100 and 1700. Whole decode steps of the gpt-oss-20b shape: 8 tokens prepacked 104 -> 85 us, 64
-// prepacked 140 -> 121, 128 from the checkpoint layout 205 -> 151; 48 tokens of 16 experts each (hidden 7168, ispp
-// 512) 726 -> 413.
+// weight it took 1100 and 1700. Whole decode steps of the gpt-oss-20b shape: 8 tokens prepacked 105 -> 87 us, 64
+// prepacked 142 -> 117, 128 from the checkpoint layout 206 -> 152; 48 tokens of 16 experts each (hidden 7168, ispp
+// 512) 728 -> 400.
 //
 // Warp roles (one persistent CTA per SM; every CTA takes a contiguous range of the (token tile,
 // feature tile) items, so that the tile's rows and scales are looked up once for many items):
