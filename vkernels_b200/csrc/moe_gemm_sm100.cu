@@ -772,7 +772,8 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 a[i] = *reinterpret_cast<const float4*>(stage + ((lane >> 3) + 4 * i) * 32 + hq);
-                a[i].x += b4.x; a[i].y += b4.y; a[i].z += b4.z; a[i].w += b4.w;   // (no bias with plain rows)
+                // plain rows leave as they are: whoever combines them (combine_rows_kernel, the ranks' reduction) adds the bias
+                if (p.raw == nullptr) { a[i].x += b4.x; a[i].y += b4.y; a[i].z += b4.z; a[i].w += b4.w; }
               }
               if (p.raw != nullptr) {   // plain partial rows, no bias, no routing weight
 #pragma unroll
