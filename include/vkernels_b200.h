@@ -243,6 +243,10 @@ int vk_cuda_moe_reset_kernel_status(void);
  * word like a GEMM kernel would. It returns by itself; nothing hangs and no real launch is
  * starved. */
 int vk_cuda_moe_test_wait_timeout(long long limit_clocks, void* stream);
+/* Test hook, host arithmetic only: the form that a layer call of this shape takes. out[4] = {1 for the
+ * fp4 form, the limit its token tiles are built with, tokens that a shared-memory slot of the
+ * gate/up GEMM holds, the same of the down GEMM} (the last two 0 for the bf16 forms). */
+int vk_cuda_moe_test_form(int M, int top_k, int EM, int block_size, int hidden, int ispp, int packed, int* out);
 
 /* Device time of the two GEMM kernels, measured with events on the launch
  * stream around up to max_calls layer calls; _end synchronises and returns the

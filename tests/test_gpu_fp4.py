@@ -59,6 +59,40 @@ def test_tile_edges(H, I, counts):
                 assert_close_bf16(y, ref, f"bf16 output {H} {I} {counts} {kw}", got_is_bf16=True)
 
 
+@pytest.mark.parametrize("M,k,E", [(4, 4, 1), (8, 4, 2), (8, 8, 3), (5, 3, 2)])
+def test_an_expert_named_twice_by_a_token(M, k, E):
+    """More rows in an expert than the batch has tokens: tiles of nine to sixteen rows, and several of them, in a batch of up
+    to eight tokens."""
+    H, I = 320, 192
+    w, A, _, _ = _problem(H, I, (M,) + (0,) * (E - 1))
+    rng = np.random.default_rng(M)
+    ids = torch.from_numpy(rng.integers(0, E, (M, k)).astype(np.int32)).to(DEV)
+    tw = torch.from_numpy((0.1 + rng.random((M, k))).astype(np.float32)).to(DEV)
+    ref = oracle_layer(A, w, ids, tw)
+    assert_close_bf16(to_np(gpu_layer(A, w, ids, tw)), ref, f"fp32 output {M} {k} {E}")
+    for y in _bf16_forms(w, A, ids, tw):
+        assert_close_bf16(y, ref, f"bf16 output {M} {k} {E}", got_is_bf16=True)
+
+
+def test_real_rows_behind_padding():
+    """A list whose blocks begin with padding: eight tokens, real rows in the last eight of sixteen."""
+    H, I, M = 320, 192, 8
+    w, A, ids, tw = _problem(H, I, (M,))
+    sids = torch.cat([torch.full((8,), M), torch.arange(M)]).to(torch.int32).to(DEV)
+    eids = torch.zeros(1, dtype=torch.int32, device=DEV)
+    act = torch.zeros((16, I), dtype=torch.bfloat16, device=DEV)
+    ref = oracle_layer(A, w, ids, tw)
+    out = torch.zeros((M, H), dtype=torch.float32, device=DEV)
+    ops.fused_moe_mxfp4_into(out, act, A, w["w13"], w["w13_scale"], w["w2"], w["w2_scale"], tw.reshape(-1), sids, eids, top_k=1)
+    y = torch.empty((M, H), dtype=torch.bfloat16, device=DEV)
+    pk = ops.prepack_weights(w["w13"], w["w13_scale"], w["w2"], w["w2_scale"])
+    ops.fused_moe_mxfp4_bf16_prepacked_into(y, act, A, pk, tw.reshape(-1), sids, eids, top_k=1)
+    torch.cuda.synchronize()
+    ops.kernel_status()
+    assert_close_bf16(to_np(out), ref, "checkpoint layout")
+    assert_close_bf16(to_np(y.float()), ref, "prepacked", got_is_bf16=True)
+
+
 def test_wide_range_rows():
     """Rows whose elements span far more than the seventeen bits of their integers, and rows near both ends of the
     bf16 range: the error stays below 2^-17 of the row's largest element times the weights' 1-norm."""

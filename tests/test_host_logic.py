@@ -11,7 +11,7 @@ import torch
 from vkernels_b200 import native_runtime as nr
 from vkernels_b200 import synthetic as syn
 from vkernels_b200.experts import StepArena
-from vkernels_b200.torch_ops import OpNotEligible, fused_moe_mxfp4, moe_align_block_size
+from vkernels_b200.torch_ops import OpNotEligible, align_em_bound, fused_moe_mxfp4, moe_align_block_size
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -59,6 +59,23 @@ def test_argument_errors_become_status_codes():
     lib.vk_set_last_error(0, b"")
     lib.vk_hip_fused_moe_mxfp4(*([one] * 9), 4, 100, 64, 1, one, one, 16, 0.0, 0, 4.0, 25.0, None, None, 16, None)
     assert lib.vk_last_error_code() == 1 and b"hidden" in lib.vk_last_error()
+
+
+@pytest.mark.parametrize("packed", [0, 1])
+@pytest.mark.parametrize("H,I", [(64, 64), (2880, 2880), (7168, 512), (32768, 64)])
+def test_token_slots_hold_the_largest_tile(H, I, packed):
+    """The fp4 form's token slots follow the limit its tile list is built with, whatever the batch: an expert may hold more
+    rows than the batch has tokens (a token that names it twice, real rows behind padding)."""
+    lib = nr.load_library()
+    out = np.zeros(4, np.int32)
+    for E in (1, 8, 128):
+        for k in (1, 4, 8):
+            for M in (*range(1, 35), 64, 255, 256, 257, 1024):
+                em = align_em_bound(M, k, E, 16)
+                assert lib.vk_cuda_moe_test_form(M, k, em, 16, H, I, packed, out.ctypes.data) == 0, nr.last_error()
+                if out[0]:
+                    assert out[1] in (16, 32) and out[2] == out[1] and out[3] == out[1], (M, k, E, out)
+    assert lib.vk_cuda_moe_test_form(8, 4, 64, 24, H, I, packed, out.ctypes.data) == 1
 
 
 def test_ops_reject_cpu_tensors_instead_of_falling_back():

@@ -25,6 +25,7 @@ void ep_reset_status();
 void ep_launch_flag_barrier(const unsigned long long* flag_bases, int world, int rank, int slot, int epoch,
                             long long limit_clocks, int* epoch_counter, cudaStream_t stream);
 void launch_wait_timeout_probe(long long limit_clocks, cudaStream_t stream);
+void sm100_test_form(int M, int top_k, int EM, int block_size, int hidden, int ispp, bool packed, int* out);
 void ep_launch_pack(const uint16_t* x, const int32_t* topk_ids, const float* topk_w, int T, int H,
                     int k, int n_shared, int world, int rank, const int32_t* expert_begin,
                     int32_t* cursor, int32_t* row_of, uint16_t* send_x, int32_t* send_ids,
@@ -294,6 +295,14 @@ int vk_cuda_moe_reset_kernel_status(void) {
 int vk_cuda_moe_test_wait_timeout(long long limit_clocks, void* stream) {
   VK_TRY
   vkc::launch_wait_timeout_probe(limit_clocks, static_cast<cudaStream_t>(stream));
+  VK_CATCH(return VK_OK, VK_RETURN_CODE)
+}
+
+/* Test hook, host arithmetic only: out[4] = {1 where the fp4 form runs, its tile limit, tokens that a shared-memory slot of
+ * the gate/up and of the down GEMM holds}. */
+int vk_cuda_moe_test_form(int M, int top_k, int EM, int block_size, int hidden, int ispp, int packed, int* out) {
+  VK_TRY
+  vkc::sm100_test_form(M, top_k, EM, block_size, hidden, ispp, packed != 0, out);
   VK_CATCH(return VK_OK, VK_RETURN_CODE)
 }
 

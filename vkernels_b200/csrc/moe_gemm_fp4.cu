@@ -895,21 +895,39 @@ digit_rows_kernel(const uint16_t* __restrict__ src, const uint16_t* const* __res
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+constexpr int kMaxSmem = 227 * 1024;
+
 template <bool GATEUP, bool PACKED>
-void launch_one(const CUtensorMap& tw, const CUtensorMap& tx8, const CUtensorMap& tx16, Fp4Params p, int max_tok,
-                cudaStream_t stream) {
-  const int max_smem = 227 * 1024;
+void launch_one(const CUtensorMap& tw, const CUtensorMap& tx8, const CUtensorMap& tx16, Fp4Params p, cudaStream_t stream) {
+  const Fp4Plan plan = fp4_plan(PACKED, p.K, p.tile_tok);
+  p.b_stages = plan.b_stages; p.b_stage_bytes = plan.b_stage_bytes; p.w_stages = plan.w_stages;
+  p.scale_bufs = plan.scale_bufs; p.scale_buf_bytes = plan.scale_buf_bytes;
+  static std::atomic<bool> configured[64];   // the attribute belongs to the device's context
+  int dev = 0;
+  VK_CUDA_CHECK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !configured[dev].load()) {
+    VK_CUDA_CHECK(cudaFuncSetAttribute(moe_gemm_fp4_kernel<GATEUP, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+    if (dev >= 0 && dev < 64) configured[dev].store(true);
+  }
+  moe_gemm_fp4_kernel<GATEUP, PACKED><<<sm_count(), n_threads(PACKED), plan.smem, stream>>>(tw, tx8, tx16, p);
+}
+
+}  // namespace
+
+Fp4Plan fp4_plan(bool packed, int K, int tile_tok) {
+  expects(tile_tok == 16 || tile_tok == 32, "fused_moe_mxfp4: the fp4 form takes tiles of up to 16 or 32 tokens");
   const int fixed = 1024 + (((int)sizeof(Bars) + 127) & ~127) + kEpiBytes + 128;
-  p.b_stage_bytes = (max_tok <= 8 ? 8 : (max_tok <= 16 ? 16 : 32)) * kDigits * 128;
-  p.scale_buf_bytes = PACKED ? 0 : (kRows * (p.K / 32) + 16 + 127) & ~127;
+  Fp4Plan p{};
+  p.b_stage_bytes = tile_tok * kDigits * 128;
+  p.scale_buf_bytes = packed ? 0 : (kRows * (K / 32) + 16 + 127) & ~127;
   // Enough scale buffers that short items do not hold the code warps back (a buffer lasts an item), four token slots of the
   // largest tiles or five of the small ones (they come from L2 with its full latency), six weight slots (96 KB an SM are what
   // HBM takes to run at its rate; three where K is so long that its scale bytes fill the rest), and what is left for tokens
   // again. The checkpoint layout wants a multiple of the teams (see the code warps).
-  const int n_kw = (p.K + kStageK - 1) / kStageK, want_w = PACKED ? kMaxW : 2 * teams(PACKED);
-  p.scale_bufs = PACKED ? 0 : std::min(kMaxSc, 2 + (kMaxW - 1) / n_kw);
-  p.b_stages = std::min(a_slots(PACKED), max_tok <= 8 ? 7 : (max_tok <= 16 || PACKED ? 5 : 4));
-  auto room = [&]() { return (max_smem - fixed - p.scale_bufs * p.scale_buf_bytes - p.b_stages * p.b_stage_bytes) / kWBytes; };
+  const int n_kw = (K + kStageK - 1) / kStageK, want_w = packed ? kMaxW : 2 * teams(packed);
+  p.scale_bufs = packed ? 0 : std::min(kMaxSc, 2 + (kMaxW - 1) / n_kw);
+  p.b_stages = tile_tok == 16 || packed ? 5 : 4;
+  auto room = [&]() { return (kMaxSmem - fixed - p.scale_bufs * p.scale_buf_bytes - p.b_stages * p.b_stage_bytes) / kWBytes; };
   while (room() < 6 && p.scale_bufs > 2) --p.scale_bufs;
   while (room() < 6 && p.b_stages > 4) --p.b_stages;
   while (room() < 6 && p.scale_bufs > 1) --p.scale_bufs;
@@ -917,23 +935,14 @@ void launch_one(const CUtensorMap& tw, const CUtensorMap& tx8, const CUtensorMap
   while (room() < 3 && p.b_stages > 1) --p.b_stages;
   expects(room() >= 3, "fused_moe_mxfp4: reduction dimension too large for shared memory");
   p.w_stages = std::min(room(), want_w);
-  if (!PACKED) p.w_stages -= p.w_stages % teams(PACKED);
-  while (p.b_stages < a_slots(PACKED) && (max_smem - fixed - p.scale_bufs * p.scale_buf_bytes - (p.b_stages + 1) * p.b_stage_bytes) / kWBytes >= p.w_stages)
+  if (!packed) p.w_stages -= p.w_stages % teams(packed);
+  while (p.b_stages < a_slots(packed) && (kMaxSmem - fixed - p.scale_bufs * p.scale_buf_bytes - (p.b_stages + 1) * p.b_stage_bytes) / kWBytes >= p.w_stages)
     ++p.b_stages;
-  const int smem = fixed + p.scale_bufs * p.scale_buf_bytes + p.b_stages * p.b_stage_bytes + p.w_stages * kWBytes;
-  static std::atomic<bool> configured[64];   // the attribute belongs to the device's context
-  int dev = 0;
-  VK_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !configured[dev].load()) {
-    VK_CUDA_CHECK(cudaFuncSetAttribute(moe_gemm_fp4_kernel<GATEUP, PACKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    if (dev >= 0 && dev < 64) configured[dev].store(true);
-  }
-  moe_gemm_fp4_kernel<GATEUP, PACKED><<<sm_count(), n_threads(PACKED), smem, stream>>>(tw, tx8, tx16, p);
+  p.smem = fixed + p.scale_bufs * p.scale_buf_bytes + p.b_stages * p.b_stage_bytes + p.w_stages * kWBytes;
+  return p;
 }
 
-}  // namespace
-
-void launch_gemm_fp4(bool gateup, bool packed, Fp4Params p, const uint8_t* planes, int EM, int max_tok, cudaStream_t stream) {
+void launch_gemm_fp4(bool gateup, bool packed, Fp4Params p, const uint8_t* planes, int EM, cudaStream_t stream) {
   p.status = sm100_status_address();
   const uint64_t half = (uint64_t)p.K / 2;
   const uint64_t xdims[3] = {half, (uint64_t)EM, kDigits}, xstr[2] = {half, half * EM};
@@ -955,9 +964,9 @@ void launch_gemm_fp4(bool gateup, bool packed, Fp4Params p, const uint8_t* plane
     tw = sm100_make_map_u8(p.w, 2, dims, str, box);
   }
   if (gateup)
-    packed ? launch_one<true, true>(tw, tx8, tx16, p, max_tok, stream) : launch_one<true, false>(tw, tx8, tx16, p, max_tok, stream);
+    packed ? launch_one<true, true>(tw, tx8, tx16, p, stream) : launch_one<true, false>(tw, tx8, tx16, p, stream);
   else
-    packed ? launch_one<false, true>(tw, tx8, tx16, p, max_tok, stream) : launch_one<false, false>(tw, tx8, tx16, p, max_tok, stream);
+    packed ? launch_one<false, true>(tw, tx8, tx16, p, stream) : launch_one<false, false>(tw, tx8, tx16, p, stream);
 }
 
 void launch_digit_rows(bool gather, const uint16_t* src, const uint16_t* const* src_rows, const int32_t* sorted_ids,

@@ -24,15 +24,24 @@ struct Fp4Params {
   const TokTile* tiles;
   const int* n_tiles;
   int store_rows;             // with out_rows: slot j's unweighted row is stored at row j of the token's block
+  int tile_tok;               // the tile list's limit (16 or 32): what a token slot holds
   int K, n_feat, n_ftiles;
   int N, top_k, w_sorted;
-  int b_stages, b_stage_bytes, w_stages, scale_bufs, scale_buf_bytes;
+  int b_stages, b_stage_bytes, w_stages, scale_bufs, scale_buf_bytes;   // (launch_gemm_fp4 fills these in)
   int activation;
   float limit, beta, linear_beta;
 };
 
-// planes: [6][EM][K / 2] digit planes of the sorted token rows (launch_digit_rows).
-void launch_gemm_fp4(bool gateup, bool packed, Fp4Params p, const uint8_t* planes, int EM, int max_tok, cudaStream_t stream);
+// Shared-memory plan of a launch for reduction length K over tiles of up to tile_tok tokens (16 or 32); throws where K does
+// not fit. A slot takes whatever tile the list may hold: how many rows an expert has is the list's matter, not the batch's -
+// a token may name an expert twice, and the real rows of a block need not be its first.
+struct Fp4Plan {
+  int b_stages, b_stage_bytes, w_stages, scale_bufs, scale_buf_bytes, smem;
+};
+Fp4Plan fp4_plan(bool packed, int K, int tile_tok);
+
+// planes: [6][EM][K / 2] digit planes of the sorted token rows (launch_digit_rows with the same tile_tok).
+void launch_gemm_fp4(bool gateup, bool packed, Fp4Params p, const uint8_t* planes, int EM, cudaStream_t stream);
 void launch_digit_rows(bool gather, const uint16_t* src, const uint16_t* const* src_rows, const int32_t* sorted_ids,
                        const int32_t* expert_ids, int block_size, int EM, int N, int top_k, int K, uint8_t* planes,
                        float* tok_scale, int32_t* inv, int max_tok, TokTile* tiles, int* n_tiles, int max_tiles,

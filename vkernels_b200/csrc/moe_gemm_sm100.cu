@@ -1415,7 +1415,7 @@ long long experts_estimate(int M, int top_k, int EM, int block_size) {
   return std::max<long long>(1, ((long long)EM - (long long)M * top_k) / (block_size - 1));
 }
 TileChoice choose_tiles(int M, int top_k, int EM, int block_size, int k_gateup, int k_down) {
-  // A token meets an expert at most once, so no expert holds more than M rows (+ padding).
+  // A token meets an expert once as a rule, so an expert holds at most M rows (+ padding); one that holds more gets more tiles.
   int max_tok = ((M + block_size - 1) / block_size) * block_size;
   max_tok = ((max_tok + 15) / 16) * 16;
   // When an expert sees a few dozen tokens at most, tiles are capped at 64 rows so that the launch
@@ -1439,13 +1439,36 @@ TileChoice choose_tiles(int M, int top_k, int EM, int block_size, int k_gateup, 
   if (!use_pair && max_tok > kMaxTok) max_tok = kMaxTok;
   return TileChoice{max_tok, use_pair};
 }
-}  // namespace
 
 // moe_gemm_fp4.cu takes tiles of up to 32 tokens. Where an expert sees eight on average or fewer, tiles end at 16 (a few
 // experts in a thousand hold more): the token slots are sized for the largest tile, and what they do not take holds weights -
 // or, with a very long reduction, its scale bytes.
-static int fp4_tile_limit(int M, int top_k, int EM, int block_size, int max_k) {
+int fp4_tile_limit(int M, int top_k, int EM, int block_size, int max_k) {
   return M <= 16 || max_k > 32768 || (long long)M * top_k <= 8 * experts_estimate(M, top_k, EM, block_size) ? 16 : 32;
+}
+
+// The form of a layer call: fp4 (small tiles) or bf16 (lone CTAs or pairs), and the limit its tile list is built with.
+struct Form {
+  bool fp4, use_pair;
+  int max_tok;
+};
+Form choose_form(int M, int top_k, int EM, int block_size, int hidden, int ispp, bool packed) {
+  const TileChoice c = choose_tiles(M, top_k, EM, block_size, hidden, ispp);
+  const bool fp4 = c.max_tok <= 64 && (small_fp4_mode() || packed);
+  return Form{fp4, c.use_pair, fp4 ? fp4_tile_limit(M, top_k, EM, block_size, std::max(hidden, ispp)) : c.max_tok};
+}
+}  // namespace
+
+// Test hook: {whether the fp4 form runs, its tile limit, tokens that a slot of the gate/up and of the down GEMM holds}.
+void sm100_test_form(int M, int top_k, int EM, int block_size, int hidden, int ispp, bool packed, int* out) {
+  expects(M > 0 && top_k > 0 && EM > 0 && block_size >= 16 && block_size % 16 == 0 && out != nullptr, "test_form: bad arguments");
+  const Form form = choose_form(M, top_k, EM, block_size, hidden, ispp, packed);
+  out[0] = form.fp4 ? 1 : 0;
+  out[1] = form.max_tok;
+  out[2] = out[3] = 0;
+  if (!form.fp4) return;
+  out[2] = fp4_plan(packed, hidden, form.max_tok).b_stage_bytes / (6 * 128);
+  out[3] = fp4_plan(packed, ispp, form.max_tok).b_stage_bytes / (6 * 128);
 }
 
 // moe_gemv.cu
@@ -1495,12 +1518,12 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
   // The number of experts is not an argument of the layer; the tensor maps
   // cover the rows of every expert id that fits an int32 row index.
   const uint64_t w13_rows_cap = (uint64_t)1 << 31;
-  const TileChoice choice = choose_tiles(M, top_k, EM, block_size, hidden, ispp);
-  const bool mx = choice.max_tok <= 64 && (small_fp4_mode() || w4);
-  const int max_tok = mx ? fp4_tile_limit(M, top_k, EM, block_size, std::max(hidden, ispp)) : choice.max_tok;
+  const Form form = choose_form(M, top_k, EM, block_size, hidden, ispp, w4);
+  const bool mx = form.fp4;
+  const int max_tok = form.max_tok;
   expects(!w4 || mx, "fused_moe_mxfp4: prepacked weights serve decode-size batches only (token tiles of up to 64 rows); "
                      "larger batches take the checkpoint-layout weights");
-  const bool use_pair = choice.use_pair;
+  const bool use_pair = form.use_pair;
   if (mx) {
     // Small tiles: the fp4 form. The tile list is built by an extra CTA of the row pre-pass.
     uint8_t* x4 = reinterpret_cast<uint8_t*>(gathered);   // digit planes of the token rows
@@ -1512,12 +1535,12 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
     Fp4Params f{};
     f.sorted_ids = sorted_ids; f.tiles = tiles; f.n_tiles = n_tiles;
     f.N = M * top_k; f.top_k = top_k; f.w_sorted = w_sorted; f.activation = activation;
-    f.limit = swiglu_limit; f.beta = beta; f.linear_beta = linear_beta;
+    f.limit = swiglu_limit; f.beta = beta; f.linear_beta = linear_beta; f.tile_tok = max_tok;
     Fp4Params p = f;
     p.w = w13; p.w_scale = w13_scale; p.x = A; p.x_rows = a_rows; p.tok_scale = scale_x; p.bias = b13; p.act = act_scratch;
     p.K = hidden; p.n_feat = ispp; p.n_ftiles = ispp / 64;
     timer_mark(0, stream);
-    launch_gemm_fp4(true, w4, p, x4, EM, std::min(max_tok, M), stream);
+    launch_gemm_fp4(true, w4, p, x4, EM, stream);
     timer_mark(1, stream);
     launch_digit_rows(false, act_scratch, nullptr, sorted_ids, expert_ids, block_size, EM, M * top_k, top_k, ispp, a4, scale_a,
                       nullptr, 0, nullptr, nullptr, 0, stream);
@@ -1525,7 +1548,7 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
     p.w = w2; p.w_scale = w2_scale; p.x = act_scratch; p.tok_scale = scale_a; p.bias = b2; p.topk_w = topk_w; p.out = out;
     p.out_rows = out_rows; p.store_rows = store_rows ? 1 : 0; p.raw = partial;
     p.K = ispp; p.n_feat = hidden; p.n_ftiles = (hidden + 127) / 128;
-    launch_gemm_fp4(false, w4, p, a4, EM, std::min(max_tok, M), stream);
+    launch_gemm_fp4(false, w4, p, a4, EM, stream);
     timer_mark(2, stream);
     if (ordered)
       combine_rows_kernel<<<dim3((unsigned)M, (unsigned)((hidden + 1023) / 1024)), 256, 0, stream>>>(partial, b2, topk_w, w_sorted, sorted_ids, expert_ids, inv, block_size, EM,

@@ -63,6 +63,7 @@ _SIGNATURES = {
     "vk_cuda_moe_kernel_status": (c_int, []),
     "vk_cuda_moe_reset_kernel_status": (c_int, []),
     "vk_cuda_moe_test_wait_timeout": (c_int, [ctypes.c_longlong, c_void_p]),
+    "vk_cuda_moe_test_form": (c_int, [c_int] * 7 + [c_void_p]),
     "vk_cuda_mxfp4_dequant_rows_path": (c_int, [c_void_p] * 3 + [c_int] * 3 + [c_void_p]),
     "vk_cuda_moe_timing_begin": (c_int, [c_int]),
     "vk_cuda_moe_timing_end": (c_int, [c_void_p] * 3),
