@@ -93,6 +93,16 @@ def test_real_rows_behind_padding():
     assert_close_bf16(to_np(y.float()), ref, "prepacked", got_is_bf16=True)
 
 
+@pytest.mark.parametrize("H,I", [(40064, 64), (40128, 64), (41792, 64), (64, 41792)])
+def test_longest_reductions(H, I):
+    """The scale bytes of an item next to three weight slots, and next to two."""
+    counts = (9, 2, 5)
+    w, A, ids, tw = _problem(H, I, counts)
+    ref = oracle_layer(A, w, ids, tw)
+    got = to_np(gpu_layer(A, w, ids, tw))
+    assert np.linalg.norm(got - ref) <= 2.0 ** -8 * np.linalg.norm(ref)   # (the bound of test_tile_edges)
+
+
 def test_wide_range_rows():
     """Rows whose elements span far more than the seventeen bits of their integers, and rows near both ends of the
     bf16 range: the error stays below 2^-17 of the row's largest element times the weights' 1-norm."""

@@ -78,6 +78,20 @@ def test_token_slots_hold_the_largest_tile(H, I, packed):
     assert lib.vk_cuda_moe_test_form(8, 4, 64, 24, H, I, packed, out.ctypes.data) == 1
 
 
+@pytest.mark.parametrize("dims", [lambda k: (k, 64), lambda k: (64, k)])
+def test_long_reductions_have_a_plan(dims):
+    """Reduction lengths up to where the scale bytes of an item fill the shared memory are served, in steps of 64: up to 41792
+    elements in batches of up to sixteen tokens, 37696 in larger ones."""
+    lib = nr.load_library()
+    out = np.zeros(4, np.int32)
+    for M, limit in ((1, 41792), (8, 41792), (16, 41792), (17, 37696), (64, 37696), (256, 37696)):
+        for K in (*range(64, limit, 1984), 32768, 32832, limit - 64, limit):
+            H, I = dims(K)
+            for packed in (0, 1):
+                rc = lib.vk_cuda_moe_test_form(M, 4, align_em_bound(M, 4, 8, 16), 16, H, I, packed, out.ctypes.data)
+                assert rc == 0 and out[0] == 1, (M, K, nr.last_error())
+
+
 def test_ops_reject_cpu_tensors_instead_of_falling_back():
     ids = torch.zeros((4, 2), dtype=torch.int32)
     with pytest.raises(OpNotEligible):

@@ -233,7 +233,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     }
     for (int i = 0; i < kMaxSc; ++i) {
       mbar_init(smem_u32(&bars->sc_full[i]), 1);
-      mbar_init(smem_u32(&bars->sc_empty[i]), 4 * kTeams);
+      mbar_init(smem_u32(&bars->sc_empty[i]), 4 * p.teams);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&bars->acc_full[i]), 1);
@@ -477,9 +477,9 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (lane == 0) mbar_arrive(smem_u32(&bars->ready[sa.slot]));
         sa.advance(kASlots);
       }
-    } else {
-      // A team takes every kTeams-th stage of the CTA's running stage sequence: its ring positions advance by
-      // kTeams, and a weight slot is released by its team alone. The weight ring's depth is a multiple of kTeams, so that
+    } else if (team < p.teams) {
+      // A team takes every teams-th stage of the CTA's running stage sequence: its ring positions advance by
+      // that, and a weight slot is released by its team alone. The weight ring's depth is a multiple of the teams, so that
       // a slot always belongs to one team: a barrier's parity tells a phase from the next one only to a waiter that has seen
       // the phase before, and copies complete out of order - the team of stage i cannot conclude from its own stages that
       // another team's load into the slot of i has landed.
@@ -490,6 +490,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const int L = 32 * i + lane;
         sf_row[i] = GATEUP ? (((L >> 3) & 1) * 64 + (L >> 4) * 8 + (L & 7)) : L;
       }
+      const int n_teams = p.teams;
       int w_slot = team, a_slot = team;
       uint32_t w_phase = 0, a_phase = 0;
       int kw = team, seq = 0;   // stage inside the item; running number of the item
@@ -502,7 +503,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const int rows_valid = GATEUP ? 128 : min(128, p.n_feat - wk.f * 128);
         if (!mbar_wait(smem_u32(&bars->sc_full[sc.slot]), sc.phase, abort_flag, 7)) break;
         const uint8_t* sc_tile = sc_smem + sc.slot * p.scale_buf_bytes;
-        for (; kw < n_kw; kw += kTeams) {
+        for (; kw < n_kw; kw += n_teams) {
           if (!codes_seen && !mbar_wait(smem_u32(&bars->w_full[w_slot]), w_phase, abort_flag, 8)) {
             ok = false;
             break;
@@ -555,14 +556,14 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
           const uint32_t slot_col = t_row + a_slot * kACols;
           tc_st32(slot_col, v);
           tc_st8(slot_col + kSfCol, sf);
-          w_slot += kTeams;
+          w_slot += n_teams;
           if (w_slot >= p.w_stages) { w_slot -= p.w_stages; w_phase ^= 1u; }
           codes_seen = mbar_test(smem_u32(&bars->w_full[w_slot]), w_phase);
           tc_wait_st();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&bars->ready[a_slot]));
-          a_slot += kTeams;
+          a_slot += n_teams;
           if (a_slot >= kASlots) { a_slot -= kASlots; a_phase ^= 1u; }
         }
         kw -= n_kw;
@@ -901,7 +902,7 @@ template <bool GATEUP, bool PACKED>
 void launch_one(const CUtensorMap& tw, const CUtensorMap& tx8, const CUtensorMap& tx16, Fp4Params p, cudaStream_t stream) {
   const Fp4Plan plan = fp4_plan(PACKED, p.K, p.tile_tok);
   p.b_stages = plan.b_stages; p.b_stage_bytes = plan.b_stage_bytes; p.w_stages = plan.w_stages;
-  p.scale_bufs = plan.scale_bufs; p.scale_buf_bytes = plan.scale_buf_bytes;
+  p.scale_bufs = plan.scale_bufs; p.scale_buf_bytes = plan.scale_buf_bytes; p.teams = plan.teams;
   static std::atomic<bool> configured[64];   // the attribute belongs to the device's context
   int dev = 0;
   VK_CUDA_CHECK(cudaGetDevice(&dev));
@@ -922,9 +923,11 @@ Fp4Plan fp4_plan(bool packed, int K, int tile_tok) {
   p.scale_buf_bytes = packed ? 0 : (kRows * (K / 32) + 16 + 127) & ~127;
   // Enough scale buffers that short items do not hold the code warps back (a buffer lasts an item), four token slots of the
   // largest tiles or five of the small ones (they come from L2 with its full latency), six weight slots (96 KB an SM are what
-  // HBM takes to run at its rate; three where K is so long that its scale bytes fill the rest), and what is left for tokens
-  // again. The checkpoint layout wants a multiple of the teams (see the code warps).
-  const int n_kw = (K + kStageK - 1) / kStageK, want_w = packed ? kMaxW : 2 * teams(packed);
+  // HBM takes to run at its rate; fewer where K is so long that its scale bytes fill the rest), and what is left for tokens
+  // again. The checkpoint layout wants a multiple of the teams (see the code warps): three, or with K beyond some 40 000, where
+  // the scale bytes leave room for two slots only, two.
+  const int n_kw = (K + kStageK - 1) / kStageK;
+  p.teams = teams(packed);
   p.scale_bufs = packed ? 0 : std::min(kMaxSc, 2 + (kMaxW - 1) / n_kw);
   p.b_stages = tile_tok == 16 || packed ? 5 : 4;
   auto room = [&]() { return (kMaxSmem - fixed - p.scale_bufs * p.scale_buf_bytes - p.b_stages * p.b_stage_bytes) / kWBytes; };
@@ -933,9 +936,10 @@ Fp4Plan fp4_plan(bool packed, int K, int tile_tok) {
   while (room() < 6 && p.scale_bufs > 1) --p.scale_bufs;
   while (room() < 6 && p.b_stages > 3) --p.b_stages;
   while (room() < 3 && p.b_stages > 1) --p.b_stages;
-  expects(room() >= 3, "fused_moe_mxfp4: reduction dimension too large for shared memory");
-  p.w_stages = std::min(room(), want_w);
-  if (!packed) p.w_stages -= p.w_stages % teams(packed);
+  if (!packed && room() < 3) p.teams = 2;
+  expects(room() >= p.teams, "fused_moe_mxfp4: reduction dimension too large for shared memory");
+  p.w_stages = std::min(room(), packed ? kMaxW : 2 * p.teams);
+  p.w_stages -= p.w_stages % p.teams;
   while (p.b_stages < a_slots(packed) && (kMaxSmem - fixed - p.scale_bufs * p.scale_buf_bytes - (p.b_stages + 1) * p.b_stage_bytes) / kWBytes >= p.w_stages)
     ++p.b_stages;
   p.smem = fixed + p.scale_bufs * p.scale_buf_bytes + p.b_stages * p.b_stage_bytes + p.w_stages * kWBytes;

@@ -27,7 +27,7 @@ struct Fp4Params {
   int tile_tok;               // the tile list's limit (16 or 32): what a token slot holds
   int K, n_feat, n_ftiles;
   int N, top_k, w_sorted;
-  int b_stages, b_stage_bytes, w_stages, scale_bufs, scale_buf_bytes;   // (launch_gemm_fp4 fills these in)
+  int b_stages, b_stage_bytes, w_stages, scale_bufs, scale_buf_bytes, teams;   // (launch_gemm_fp4 fills these in)
   int activation;
   float limit, beta, linear_beta;
 };
@@ -36,7 +36,7 @@ struct Fp4Params {
 // not fit. A slot takes whatever tile the list may hold: how many rows an expert has is the list's matter, not the batch's -
 // a token may name an expert twice, and the real rows of a block need not be its first.
 struct Fp4Plan {
-  int b_stages, b_stage_bytes, w_stages, scale_bufs, scale_buf_bytes, smem;
+  int b_stages, b_stage_bytes, w_stages, scale_bufs, scale_buf_bytes, teams, smem;
 };
 Fp4Plan fp4_plan(bool packed, int K, int tile_tok);
 
