@@ -179,6 +179,40 @@ def test_router_logits_tensor_core_kernel(T, E, H):
     assert float(np.abs(to_np(lg) - exact).max()) <= noise + 2e-6
 
 
+@pytest.mark.parametrize("T,E,H", [(65, 256, 2880), (129, 256, 7168), (333, 256, 2880), (512, 256, 1536)])
+def test_router_logits_of_a_token_do_not_depend_on_its_batch(T, E, H):
+    """65 to 512 tokens: bit for bit the logits of smaller batches, and at least as close to the float64 dot products as the
+    oracle's sequential fp32 sums."""
+    cfg = syn.scaled(syn.CONFIGS["c2"], H=H, E=E)
+    r = syn.make_router(cfg, device=DEV)
+    A = syn.make_activations(cfg, T, device=DEV)
+    lg = ops.router_logits(A, r["wr"])
+    for t0 in (*range(0, T - 40, 40), T - 40):
+        assert torch.equal(lg[t0:t0 + 40], ops.router_logits(A[t0:t0 + 40].contiguous(), r["wr"]))
+    exact = A.float().cpu().numpy().astype(np.float64) @ to_np(r["wr"]).astype(np.float64).T
+    noise = float(np.abs(oracle.router_logits(bf16_to_u16(A), to_np(r["wr"])) - exact).max())
+    assert float(np.abs(to_np(lg) - exact).max()) <= noise + 2e-6
+
+
+@pytest.mark.parametrize("T,E,H", [(128, 128, 2880), (333, 128, 2880), (512, 256, 2880)])
+def test_router_logits_captured_on_a_stream_without_scratch(T, E, H):
+    """Up to 512 tokens the router takes no scratch: a stream that never ran the library can capture it, and the replay gives
+    the eager call's logits."""
+    cfg = syn.scaled(syn.CONFIGS["c2"], H=H, E=E)
+    r = syn.make_router(cfg, device=DEV)
+    A = syn.make_activations(cfg, T, device=DEV)
+    eager = ops.router_logits(A, r["wr"])
+    out = torch.empty_like(eager)
+    torch.cuda.synchronize()
+    live = nr.load_library().vk_cuda_moe_workspace_live_bytes()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream(device=DEV)):
+        ops.router_logits(A, r["wr"], out=out)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager) and nr.load_library().vk_cuda_moe_workspace_live_bytes() == live
+
+
 def test_routing_zipf_logits():
     cfg = syn.CONFIGS["c4"]
     _check_route(cfg, 4096, logits=syn.make_zipf_logits(cfg, 4096, device=DEV))

@@ -34,8 +34,6 @@ inline void expects(bool ok, const char* msg) {
 // No call synchronises the device or frees memory. While `stream` is being captured nothing can
 // be allocated: the call throws std::invalid_argument (reserve before capturing).
 void* workspace_get(size_t bytes, cudaStream_t stream);
-// The same, but a null pointer instead of the exception.
-void* workspace_try(size_t bytes, cudaStream_t stream);
 
 // Number of SMs of the current device.
 int sm_count();

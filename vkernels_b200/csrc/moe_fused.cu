@@ -79,7 +79,7 @@ int sm_count() {
   return v;
 }
 
-void* workspace_try(size_t bytes, cudaStream_t stream) {
+void* workspace_get(size_t bytes, cudaStream_t stream) {
   int dev = 0;
   VK_CUDA_CHECK(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(g_ws_mutex);
@@ -89,7 +89,9 @@ void* workspace_try(size_t bytes, cudaStream_t stream) {
   if (mine != nullptr && mine->bytes >= bytes) return mine->ptr;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   VK_CUDA_CHECK(cudaStreamIsCapturing(stream, &cap));
-  if (cap != cudaStreamCaptureStatusNone) return nullptr;
+  expects(cap == cudaStreamCaptureStatusNone,
+          "fused_moe_mxfp4: the workspace of this stream is too small and the stream is being "
+          "captured; call vk_cuda_moe_reserve_workspace_on(bytes, stream) before the capture");
   const size_t want = (bytes + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
   void* p = nullptr;
   VK_CUDA_CHECK(cudaMalloc(&p, want));
@@ -100,13 +102,6 @@ void* workspace_try(size_t bytes, cudaStream_t stream) {
   } else {
     g_ws_live.push_back(WsBlock{dev, stream, p, want});
   }
-  return p;
-}
-
-void* workspace_get(size_t bytes, cudaStream_t stream) {
-  void* p = workspace_try(bytes, stream);
-  expects(p != nullptr, "fused_moe_mxfp4: the workspace of this stream is too small and the stream is being "
-                        "captured; call vk_cuda_moe_reserve_workspace_on(bytes, stream) before the capture");
   return p;
 }
 

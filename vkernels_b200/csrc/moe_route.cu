@@ -607,17 +607,12 @@ bool router_tc_mode() {
   return on;
 }
 
-// Returns false, with nothing launched, where the call would need scratch that a capture does not let it allocate.
-bool launch_router_tc(const uint16_t* x, const float* wr, float* logits, int T, int H, int E, cudaStream_t st) {
+void launch_router_tc(const uint16_t* x, const float* wr, float* logits, int T, int H, int E, cudaStream_t st) {
   const int tiles = (T + 127) / 128, chunks = H / 64;
-  // K slices of at least four chunks: up to eight, and more while the logits are so few that a plane of them costs less than
-  // the chunks it takes off every CTA
-  int z = std::max(1, std::min(std::min(tiles <= 4 ? 32 : 8, chunks / 4), sm_count() / tiles));
+  int z = std::max(1, std::min(std::min(8, chunks / 4), sm_count() / tiles));
   const size_t n = (size_t)T * E, n_w = (size_t)E * H;
   const size_t w_bytes = (3 * n_w * sizeof(uint16_t) + 1023) & ~size_t(1023);
-  uint8_t* ws = static_cast<uint8_t*>(workspace_try(4096 + w_bytes + (z > 1 ? (size_t)z * n * sizeof(float) : 0), st));
-  if (ws == nullptr) return false;
-  ws += 4096;
+  uint8_t* ws = static_cast<uint8_t*>(workspace_get(4096 + w_bytes + (z > 1 ? (size_t)z * n * sizeof(float) : 0), st)) + 4096;
   uint16_t* w_planes = reinterpret_cast<uint16_t*>(ws);
   float* planes = z > 1 ? reinterpret_cast<float*>(ws + w_bytes) : logits;
   split_router_weight_kernel<<<(unsigned)((n_w + 255) / 256), 256, 0, st>>>(wr, n_w, w_planes);
@@ -637,7 +632,6 @@ bool launch_router_tc(const uint16_t* x, const float* wr, float* logits, int T, 
   router_logits_tc_kernel<<<dim3((unsigned)tiles, (unsigned)z), 192, smem, st>>>(map_x, map_w, planes, T, H, E, stages,
                                                                               sm100_status_address());
   if (z > 1) sum_planes_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, st>>>(planes, z, n, logits);
-  return true;
 }
 }  // namespace
 
@@ -647,22 +641,18 @@ void router_logits(const uint16_t* x, const float* wr, float* logits, int T, int
   if (T == 0) return;
   expects(x && wr && logits, "router_logits: null buffer");
   const bool aligned16 = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(wr) & 15u) == 0;
-  const bool tc = router_tc_mode() && H % 64 == 0 && E % 16 == 0 && E <= 256 && aligned16;
-  // Up to 512 tokens the dot-product kernels read the weight row again for every token. That is cheaper than the tensor-core
-  // kernel's three launches (15 us at 333 x 128 x 2880, where they take 53) up to some 32 million products (8 us at 128 x
-  // 32 x 2880), and up to 64 tokens in any case: there the weight's own split costs as much (21 us both at 32 x 256 x 7168).
-  if (tc && T > 64 && T <= 512 && (long long)T * E * H > (32ll << 20) &&
-      launch_router_tc(x, wr, logits, T, H, E, static_cast<cudaStream_t>(stream))) {
-  } else if ((long long)T * E <= 8192 && T <= 65535 && H % 8 == 0 && aligned16) {
+  // Up to 512 tokens: dot products. They take no scratch, so that a call is accepted on any stream, captured or not, and gives
+  // the same logits there. (The tensor-core kernel, whose scratch a capture cannot allocate, is faster from some hundred tokens
+  // on - 12.6 us for 31.2 at 333 x 128 x 2880, 12.2 for 15.1 at 128 x 128 x 2880, inputs in L2 - but a route that falls back where the scratch
+  // is missing gives logits that depend on what ran on the stream before.)
+  if ((long long)T * E <= 8192 && T <= 65535 && H % 8 == 0 && aligned16) {
     router_logits_cta_kernel<<<dim3((unsigned)E, (unsigned)T), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, wr, logits, H, E);
   } else if (T <= 512 && H % 8 == 0 && aligned16) {   // 8- and 16-byte loads of whole rows
     const long long pairs = (long long)T * E;
     router_logits_warp_kernel<<<(unsigned)((pairs + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         x, wr, logits, T, H, E);
-  } else if (tc) {
-    expects(launch_router_tc(x, wr, logits, T, H, E, static_cast<cudaStream_t>(stream)),
-            "router_logits: the workspace of this stream is too small and the stream is being captured; call "
-            "vk_cuda_moe_reserve_workspace_on(bytes, stream) before the capture");
+  } else if (router_tc_mode() && H % 64 == 0 && E % 16 == 0 && E <= 256 && aligned16) {
+    launch_router_tc(x, wr, logits, T, H, E, static_cast<cudaStream_t>(stream));
   } else if (H % 8 == 0 && aligned16) {
     // the attribute belongs to the device's context: once per device
     static std::atomic<bool> configured_dev[64];
