@@ -226,6 +226,13 @@ int vk_cuda_moe_get_impl(void);
  * vk_cuda_moe_release_workspaces frees all blocks of the current device: only when none of the
  * library's work is pending and no captured graph using them will be replayed. */
 size_t vk_cuda_moe_workspace_bytes(int max_EM, int hidden, int ispp, int n_local_experts, int N);
+/* A call's scratch follows the form it runs, and the function above covers them all for max_EM rows. This one knows the batches:
+ * bytes with which everything fits that a layer of n_local_experts experts and top_k slots a token does with up to max_tokens
+ * tokens - router (n_router experts scored; 0 without one), alignment, and the layer with EM at the alignment's host bound,
+ * min(N, experts) * block_size + the other rows rounded up, N = tokens * top_k; up to ordered_tokens tokens also the bf16
+ * result forms. 0 for bad arguments (vk_last_error). */
+size_t vk_cuda_moe_workspace_bytes_upto(int max_tokens, int top_k, int n_local_experts, int hidden, int ispp, int block_size,
+                                        int ordered_tokens, int n_router);
 int vk_cuda_moe_reserve_workspace(size_t bytes);
 int vk_cuda_moe_reserve_workspace_on(size_t bytes, void* stream);
 int vk_cuda_moe_release_workspaces(void);

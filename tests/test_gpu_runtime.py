@@ -114,3 +114,24 @@ def test_capture_refuses_to_allocate_and_replay_survives_growth():
     ref = oracle_layer(A, w, torch.from_numpy(ids_np), torch.from_numpy(tw_np))
     ok = margin > 2e-5
     assert_close_bf16(to_np(y.float())[ok], ref[ok], "replay after growth", got_is_bf16=True)
+
+
+def test_a_layer_reserves_for_every_batch_of_its_budget():
+    """No batch up to the token budget, in whichever form, makes the library allocate after the layer has been built; a layer
+    with a router for more than 512 tokens reserves the router's scratch too."""
+    lib = nr.load_library()
+    for cfg, T in ((syn.scaled(syn.CONFIGS["c0"], H=256, I=128, E=8, top_k=2), 600),
+                   (syn.scaled(syn.CONFIGS["c0"], H=512, I=64, E=256, top_k=1), 1024),
+                   (syn.scaled(syn.CONFIGS["c0"], H=64, I=512, E=4, top_k=2), 300)):
+        w, A, r = make_case(cfg, T, backend="torch")
+        with torch.cuda.stream(torch.cuda.Stream()):
+            layer = layer_from_config(cfg, w, r, max_tokens=T, prepack=True)
+            live = lib.vk_cuda_moe_workspace_live_bytes()
+            for t in (1, 5, 8, 33, 64, 192, 200, 256, 257, 300, 513, 600, 1024):
+                if t <= T:
+                    ids, tw = layer.route(A[:t])
+                    layer.experts_fp32(A[:t], ids, tw)
+                    layer.forward(A[:t])
+                    assert lib.vk_cuda_moe_workspace_live_bytes() == live, t
+            torch.cuda.synchronize()
+            ops.kernel_status()

@@ -92,6 +92,26 @@ def test_long_reductions_have_a_plan(dims):
                 assert rc == 0 and out[0] == 1, (M, K, nr.last_error())
 
 
+@pytest.mark.parametrize("T,k,E,H,I", [(16384, 9, 257, 7168, 2048), (8192, 4, 128, 2880, 2880), (300, 2, 8, 64, 1024), (40, 16, 256, 7168, 512)])
+def test_layer_scratch_follows_the_form(T, k, E, H, I):
+    """The scratch that a layer reserves holds every batch up to its budget - gathered bf16 rows in the large forms, digit planes
+    in the small one, partial rows in the ordered one - and no digit planes for batches that have none: at most two bytes an
+    element of the token and activation rows of the largest batch, or what the ordered batches take."""
+    lib = nr.load_library()
+    out = np.zeros(4, np.int32)
+    got = lib.vk_cuda_moe_workspace_bytes_upto(T, k, E, H, I, 16, 256, 0)
+    rows = lambda M: align_em_bound(M, k, E, 16)
+    for M in sorted({*range(1, min(T, 400)), T // 2, T - 1, T}):
+        em = rows(M)
+        assert lib.vk_cuda_moe_test_form(M, k, em, 16, H, I, 0, out.ctypes.data) == 0
+        need = 3 * max(H, I) * em if out[0] else 2 * H * em
+        if M <= 256:
+            need = max(need, (4 * H + 3 * I) * em)
+        assert got >= need, M
+    assert got <= max(2 * (H + I) * rows(T), (4 * H + 3 * I) * rows(min(T, 256))) + 64 * rows(T) + (1 << 16)
+    assert lib.vk_cuda_moe_workspace_bytes_upto(T, 0, E, H, I, 16, 256, 0) == 0
+
+
 def test_ops_reject_cpu_tensors_instead_of_falling_back():
     ids = torch.zeros((4, 2), dtype=torch.int32)
     with pytest.raises(OpNotEligible):

@@ -82,6 +82,7 @@ void set_error(int code, const char* msg) {
   }
 #define VK_RETURN_CODE(c) return (c)
 #define VK_RETURN_VOID(c) return
+#define VK_RETURN_ZERO(c) return 0
 
 namespace {
 // RAII device buffer for the host-pointer entry points.
@@ -238,6 +239,13 @@ int vk_cuda_moe_get_impl(void) { return static_cast<int>(vkc::get_moe_impl()); }
 
 size_t vk_cuda_moe_workspace_bytes(int max_EM, int hidden, int ispp, int n_local_experts, int N) {
   return vkc::workspace_bytes_required(max_EM, hidden, ispp, n_local_experts, N);
+}
+size_t vk_cuda_moe_workspace_bytes_upto(int max_tokens, int top_k, int n_local_experts, int hidden, int ispp, int block_size,
+                                        int ordered_tokens, int n_router) {
+  size_t n = 0;
+  VK_TRY
+  n = vkc::workspace_bytes_upto(max_tokens, top_k, n_local_experts, hidden, ispp, block_size, ordered_tokens, n_router);
+  VK_CATCH(return n, VK_RETURN_ZERO)
 }
 int vk_cuda_moe_reserve_workspace(size_t bytes) {
   VK_TRY

@@ -1,6 +1,7 @@
 // moe_fused.cu - host launchers: argument contract, workspace, dispatch.
 #include "moe_fused.hpp"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -27,6 +28,9 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
                       const RowPtrs* rows, uint16_t* y_bf16, bool w4);
 size_t sm100_workspace_bytes(int EM, int hidden, int ispp);
 size_t sm100_workspace_bytes_ordered(int EM, int hidden, int ispp, int N);
+size_t sm100_workspace_bytes_upto(int max_tokens, int top_k, int n_experts, int hidden, int ispp, int block_size,
+                                  int ordered_tokens);
+size_t router_scratch_bytes_upto(int max_tokens, int H, int E);   // moe_route.cu
 
 // ---------------------------------------------------------------------------
 // implementation switch
@@ -136,11 +140,27 @@ size_t workspace_live_bytes() {
   return n;
 }
 
+namespace {
+size_t align_scratch_bytes(int n_local_experts, int N) {
+  return ((size_t)((N + 1023) / 1024) + 1) * (size_t)(n_local_experts > 0 ? n_local_experts : 1) * 4;
+}
+}  // namespace
+
 size_t workspace_bytes_required(int max_EM, int hidden, int ispp, int n_local_experts, int N) {
-  const size_t align_bytes =
-      ((size_t)((N + 1023) / 1024) + 1) * (size_t)(n_local_experts > 0 ? n_local_experts : 1) * 4;
+  const size_t align_bytes = align_scratch_bytes(n_local_experts, N);
   const size_t gemm_bytes = sm100_workspace_bytes(max_EM, hidden, ispp);
   return (align_bytes > gemm_bytes ? align_bytes : gemm_bytes) + 4096;
+}
+
+size_t workspace_bytes_upto(int max_tokens, int top_k, int n_local_experts, int hidden, int ispp, int block_size,
+                            int ordered_tokens, int n_router) {
+  expects(max_tokens >= 0 && top_k > 0 && n_local_experts > 0 && hidden > 0 && ispp > 0, "workspace_bytes_upto: bad dimensions");
+  expects(block_size >= 16 && block_size % 16 == 0, "workspace_bytes_upto: block_size must be a multiple of 16");
+  expects((long long)max_tokens * top_k + (long long)n_local_experts * block_size < (1ll << 30), "workspace_bytes_upto: batch too large");
+  size_t b = sm100_workspace_bytes_upto(max_tokens, top_k, n_local_experts, hidden, ispp, block_size, ordered_tokens);
+  b = std::max(b, align_scratch_bytes(n_local_experts, max_tokens * top_k));
+  if (n_router > 0) b = std::max(b, router_scratch_bytes_upto(max_tokens, hidden, n_router));
+  return b + 4096;
 }
 
 // ---------------------------------------------------------------------------

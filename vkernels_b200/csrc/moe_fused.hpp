@@ -192,6 +192,12 @@ void route_align_small(const float* logits, const float* bias, int T, int E, int
 // allocation is impossible and the call fails with std::invalid_argument: reserve first.
 size_t workspace_bytes_required(int max_EM, int hidden, int ispp, int n_local_experts,
                                 int N);
+// Scratch for everything that a layer of n_local_experts experts, top_k slots a token, does with up to max_tokens tokens:
+// router (n_router experts scored; 0 without one), alignment, the layer with EM at the alignment's host bound; up to
+// ordered_tokens tokens also the ordered form. A call's scratch follows the form it runs, which the two functions above do not
+// know: they take the larger one for max_EM rows.
+size_t workspace_bytes_upto(int max_tokens, int top_k, int n_local_experts, int hidden, int ispp, int block_size,
+                            int ordered_tokens, int n_router);
 void reserve_workspace(size_t bytes, void* stream = nullptr);
 void release_workspaces();
 size_t workspace_live_bytes();

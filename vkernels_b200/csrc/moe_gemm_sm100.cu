@@ -1134,28 +1134,36 @@ TokMaps token_maps(const void* rows, int K, int EM, bool pair) {
 
 int max_tok_tiles(int EM) { return EM / 16 + 1; }
 
-// gathered: [EM, hidden] bf16 rows, or - fp4 form - the six digit planes of those rows [6][EM, hidden / 2] and, behind
-// them, of the activation rows [6][EM, ispp / 2]; scales: one fp32 per row each.
-// ordered = the bf16-output form: + the inverse permutation [N] and the fp32 partial rows
-// [EM, hidden] of the down GEMM.
+// Scratch of one layer call. bf16 forms: the gathered rows [EM, hidden] bf16. fp4 form: the six digit planes of the token rows
+// [6][EM, hidden / 2] and of the activation rows [6][EM, ispp / 2], one fp32 scale per row each. The token planes are dead when
+// the activation planes are written (the gate/up GEMM lies between them on the stream), so the two share their place -
+// or, in the ordered form, the token planes lie where the down GEMM puts its partial rows later.
+// ordered = the bf16-output form: + the inverse permutation [N] and the fp32 partial rows [EM, hidden] of the down GEMM.
 struct WsLayout {
-  size_t tiles_off, count_off, gathered_off, act4_off, scale_x_off, scale_a_off, inv_off, partial_off, total;
+  size_t tiles_off, count_off, rows_off, act4_off, scale_x_off, scale_a_off, inv_off, partial_off, total;
 };
-WsLayout ws_layout(int EM, int hidden, int ispp, bool ordered = false, int N = 0) {
+WsLayout ws_layout(bool fp4, int EM, int hidden, int ispp, bool ordered = false, int N = 0) {
   WsLayout l{};
   size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = off;
+    off = (off + bytes + 1023) & ~size_t(1023);
+    return at;
+  };
   l.count_off = off;  off += 256;
-  l.tiles_off = off;  off += (size_t)max_tok_tiles(EM) * sizeof(TokTile);
-  off = (off + 1023) & ~size_t(1023);
-  l.gathered_off = off;  off += (size_t)EM * hidden * 3;
-  l.act4_off = off;  off += (size_t)EM * ispp * 3;
-  l.scale_x_off = off;  off += (size_t)EM * sizeof(float);
-  l.scale_a_off = off;  off += (size_t)EM * sizeof(float);
-  off = (off + 1023) & ~size_t(1023);
+  l.tiles_off = take((size_t)max_tok_tiles(EM) * sizeof(TokTile));
   if (ordered) {
-    l.inv_off = off;  off += (size_t)N * sizeof(int32_t);
-    off = (off + 1023) & ~size_t(1023);
-    l.partial_off = off;  off += (size_t)EM * hidden * sizeof(float);
+    l.inv_off = take((size_t)N * sizeof(int32_t));
+    l.partial_off = take((size_t)EM * hidden * sizeof(float));
+  }
+  const size_t x4 = (size_t)EM * hidden * 3, a4 = (size_t)EM * ispp * 3;
+  if (!fp4) {
+    l.rows_off = take((size_t)EM * hidden * sizeof(uint16_t));
+  } else {
+    l.scale_x_off = take((size_t)EM * sizeof(float));
+    l.scale_a_off = take((size_t)EM * sizeof(float));
+    l.rows_off = ordered ? l.partial_off : off;
+    l.act4_off = take(ordered ? a4 : std::max(x4, a4));
   }
   l.total = off;
   return l;
@@ -1266,8 +1274,13 @@ void launch_gemm(const CUtensorMap& tw, const TokMaps& tb, GemmParams p,
 
 }  // namespace
 
-size_t sm100_workspace_bytes(int EM, int hidden, int ispp) { return ws_layout(EM, hidden, ispp).total; }
-size_t sm100_workspace_bytes_ordered(int EM, int hidden, int ispp, int N) { return ws_layout(EM, hidden, ispp, true, N).total; }
+// What a call on EM sorted rows may take, whichever form it runs.
+size_t sm100_workspace_bytes(int EM, int hidden, int ispp) {
+  return std::max(ws_layout(false, EM, hidden, ispp).total, ws_layout(true, EM, hidden, ispp).total);
+}
+size_t sm100_workspace_bytes_ordered(int EM, int hidden, int ispp, int N) {
+  return std::max(ws_layout(false, EM, hidden, ispp, true, N).total, ws_layout(true, EM, hidden, ispp, true, N).total);
+}
 
 // Sizes of the prepacked form of one weight set. which = 0: w13 [E, 2 * ispp, hidden / 2];
 // 1: w2 [E, hidden, ispp / 2]. The code buffer carries 128 rows + 64 bytes of zero padding: a
@@ -1459,6 +1472,24 @@ Form choose_form(int M, int top_k, int EM, int block_size, int hidden, int ispp,
 }
 }  // namespace
 
+// Scratch with which every layer call of up to max_tokens tokens fits whose EM is the host bound of its alignment
+// (min(N, experts) experts with one row each, the other rows in one more), in the fp32 form and, up to ordered_tokens, in
+// the ordered one.
+size_t sm100_workspace_bytes_upto(int max_tokens, int top_k, int n_experts, int hidden, int ispp, int block_size,
+                                  int ordered_tokens) {
+  size_t most = 0;
+  for (int M = 1; M <= max_tokens; ++M) {
+    const long long N = (long long)M * top_k, head = std::min<long long>(N, n_experts);
+    const int EM = (int)(head * block_size + (N - head + block_size - 1) / block_size * block_size);
+    const bool fp4 = choose_form(M, top_k, EM, block_size, hidden, ispp, false).fp4;
+    most = std::max(most, ws_layout(fp4, EM, hidden, ispp).total);
+    if (M <= ordered_tokens) most = std::max(most, ws_layout(fp4, EM, hidden, ispp, true, (int)N).total);
+    // (prepacked weights run the fp4 form even where VK_MOE_SMALL keeps the others off it)
+    if (M <= ordered_tokens) most = std::max(most, ws_layout(true, EM, hidden, ispp, true, (int)N).total);
+  }
+  return most;
+}
+
 // Test hook: {whether the fp4 form runs, its tile limit, tokens that a slot of the gate/up and of the down GEMM holds}.
 void sm100_test_form(int M, int top_k, int EM, int block_size, int hidden, int ispp, bool packed, int* out) {
   expects(M > 0 && top_k > 0 && EM > 0 && block_size >= 16 && block_size % 16 == 0 && out != nullptr, "test_form: bad arguments");
@@ -1496,11 +1527,15 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
   // y_bf16 != nullptr: the down GEMM leaves plain partial rows and an ordered combine writes the
   // bf16 result (no atomics, no fp32 output buffer to zero and convert)
   const bool ordered = y_bf16 != nullptr;
-  const WsLayout l = ws_layout(EM, hidden, ispp, ordered, M * top_k);
+  const Form form = choose_form(M, top_k, EM, block_size, hidden, ispp, w4);
+  const bool mx = form.fp4;
+  expects(!w4 || mx, "fused_moe_mxfp4: prepacked weights serve decode-size batches only (token tiles of up to 64 rows); "
+                     "larger batches take the checkpoint-layout weights");
+  const WsLayout l = ws_layout(mx, EM, hidden, ispp, ordered, M * top_k);
   uint8_t* ws = static_cast<uint8_t*>(workspace_get(l.total, stream));
   TokTile* tiles = reinterpret_cast<TokTile*>(ws + l.tiles_off);
   int* n_tiles = reinterpret_cast<int*>(ws + l.count_off);
-  uint16_t* gathered = reinterpret_cast<uint16_t*>(ws + l.gathered_off);
+  uint16_t* gathered = reinterpret_cast<uint16_t*>(ws + l.rows_off);
   int32_t* inv = ordered ? reinterpret_cast<int32_t*>(ws + l.inv_off) : nullptr;
   float* partial = ordered ? reinterpret_cast<float*>(ws + l.partial_off) : nullptr;
 
@@ -1518,11 +1553,7 @@ void launch_moe_sm100(const uint16_t* A, const uint8_t* w13, const uint8_t* w13_
   // The number of experts is not an argument of the layer; the tensor maps
   // cover the rows of every expert id that fits an int32 row index.
   const uint64_t w13_rows_cap = (uint64_t)1 << 31;
-  const Form form = choose_form(M, top_k, EM, block_size, hidden, ispp, w4);
-  const bool mx = form.fp4;
   const int max_tok = form.max_tok;
-  expects(!w4 || mx, "fused_moe_mxfp4: prepacked weights serve decode-size batches only (token tiles of up to 64 rows); "
-                     "larger batches take the checkpoint-layout weights");
   const bool use_pair = form.use_pair;
   if (mx) {
     // Small tiles: the fp4 form. The tile list is built by an extra CTA of the row pre-pass.
@@ -1617,11 +1648,11 @@ void launch_moe_stage_gemm(int which, const uint16_t* rows_in, const uint8_t* w,
   expects(rows_in && w && w_scale && sorted_ids && expert_ids && raw, "moe stage: buffers must not be null");
   expects(aligned16(rows_in) && aligned16(w) && aligned16(w_scale) && aligned16(raw),
           "moe stage: buffers must be 16-byte aligned");
-  const WsLayout l = ws_layout(EM, which == 0 ? k_full : 64, 0);
+  const WsLayout l = ws_layout(false, EM, which == 0 ? k_full : 64, 0);
   uint8_t* ws = static_cast<uint8_t*>(workspace_get(l.total, stream));
   TokTile* tiles = reinterpret_cast<TokTile*>(ws + l.tiles_off);
   int* n_tiles = reinterpret_cast<int*>(ws + l.count_off);
-  uint16_t* gathered = reinterpret_cast<uint16_t*>(ws + l.gathered_off);
+  uint16_t* gathered = reinterpret_cast<uint16_t*>(ws + l.rows_off);
   const TileChoice choice = choose_tiles(M, top_k, EM, block_size, k_shard, k_shard);
   build_tiles_kernel<<<1, 1024, 0, stream>>>(expert_ids, EM / block_size, block_size, choice.max_tok, tiles,
                                              n_tiles, max_tok_tiles(EM));

@@ -635,6 +635,13 @@ void launch_router_tc(const uint16_t* x, const float* wr, float* logits, int T, 
 }
 }  // namespace
 
+// Upper bound of what router_logits takes for up to max_tokens tokens: the weight's three bf16 planes and the K slices' planes of
+// logits, of which there are as many as leave each of the 148 SMs one tile of up to 128 tokens, or one.
+size_t router_scratch_bytes_upto(int max_tokens, int H, int E) {
+  if (max_tokens <= 512) return 0;
+  return 4096 + (size_t)E * H * 6 + 1024 + ((size_t)max_tokens + 148 * 128) * E * sizeof(float);
+}
+
 void router_logits(const uint16_t* x, const float* wr, float* logits, int T, int H, int E,
                    void* stream) {
   expects(T >= 0 && H > 0 && E > 0, "router_logits: bad dimensions");

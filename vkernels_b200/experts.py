@@ -130,14 +130,11 @@ class FusedMoEMxfp4:
     TINY_SLOTS = 12
 
     def _workspace_bytes(self) -> int:
-        T = self.max_tokens
-        lib = nr.load_library()
-        plain = lib.vk_cuda_moe_workspace_bytes(self._em_bound(T), self.hidden, self.ispp, self.n_experts_total,
-                                                T * self.slots)
-        Ts = min(T, self.ORDERED_COMBINE_TOKENS)
-        small = lib.vk_cuda_moe_workspace_bytes_bf16(self._em_bound(Ts), self.hidden, self.ispp, self.n_experts_total,
-                                                     Ts * self.slots)
-        return max(plain, small)
+        n = nr.load_library().vk_cuda_moe_workspace_bytes_upto(
+            self.max_tokens, self.slots, self.n_experts_total, self.hidden, self.ispp, self.block_size, self.ORDERED_COMBINE_TOKENS,
+            0 if self.router_weight is None else self.n_router)
+        ops.require(n > 0, f"workspace_bytes_upto: {nr.last_error()}")
+        return n
 
     def _reserve(self) -> None:
         """Everything a step needs, allocated once: the library scratch of the current stream and

@@ -56,6 +56,7 @@ _SIGNATURES = {
     "vk_cuda_moe_set_impl": (c_int, [c_int]),
     "vk_cuda_moe_get_impl": (c_int, []),
     "vk_cuda_moe_workspace_bytes": (c_size_t, [c_int] * 5),
+    "vk_cuda_moe_workspace_bytes_upto": (c_size_t, [c_int] * 8),
     "vk_cuda_moe_reserve_workspace": (c_int, [c_size_t]),
     "vk_cuda_moe_reserve_workspace_on": (c_int, [c_size_t, c_void_p]),
     "vk_cuda_moe_release_workspaces": (c_int, []),
