@@ -47,7 +47,7 @@ void launch_digit_rows(bool gather, const uint16_t* src, const uint16_t* const* 
                        float* tok_scale, int32_t* inv, int max_tok, TokTile* tiles, int* n_tiles, int max_tiles,
                        cudaStream_t stream);
 
-// moe_gemm_sm100.cu: a cached byte tensor map (128-byte swizzle, boxes 128 bytes wide; dims and box
+// moe_gemm_sm100.cu: a byte tensor map (128-byte swizzle, boxes 128 bytes wide; dims and box
 // innermost first, strides of the outer dimensions in bytes) and the device address of the status word.
 CUtensorMap sm100_make_map_u8(const void* ptr, int rank, const uint64_t* dims, const uint64_t* strides, const uint32_t* box);
 int* sm100_status_address();
