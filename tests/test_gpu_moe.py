@@ -302,6 +302,24 @@ def test_bf16_form_with_ordered_combine(name, T):
     assert_close_bf16(got if tokens is None else got[tokens], ref, f"bf16 form {name} T={T}", got_is_bf16=True)
 
 
+@pytest.mark.parametrize("ids", [[[2, 2, 2, 2]], [[1, 0, 1]], [[0, 3, 3, 0], [3, 3, 1, 3], [-1, 2, -1, 2]], [[1] * 12]])
+def test_flat_form_adds_every_slot_of_a_repeated_expert(ids):
+    """A token that names an expert more than once: every slot counts, with its own routing weight."""
+    cfg = syn.scaled(syn.CONFIGS["c0"], H=256, I=128, E=4)
+    ids = torch.tensor(ids, dtype=torch.int32, device=DEV)
+    T, k = ids.shape
+    w, A, _ = make_case(cfg, T, backend="torch")
+    rng = np.random.default_rng(k)
+    tw = torch.from_numpy((0.1 + rng.random((T, k))).astype(np.float32)).to(DEV)
+    b2 = torch.from_numpy(rng.standard_normal((cfg.E, cfg.H)).astype(np.float32)).to(DEV)
+    sids, eids, _ = ops.moe_align_block_size(ids, cfg.E, 16)
+    act = torch.zeros((sids.numel(), cfg.I), dtype=torch.bfloat16, device=DEV)
+    y = torch.empty((T, cfg.H), dtype=torch.bfloat16, device=DEV)
+    ops.fused_moe_mxfp4_bf16_into(y, act, A, w["w13"], w["w13_scale"], w["w2"], w["w2_scale"], tw.reshape(-1), sids, eids, top_k=k, b2=b2)
+    torch.cuda.synchronize()
+    assert_close_bf16(to_np(y.float()), oracle_layer(A, w, ids, tw, b2=to_np(b2)), f"flat form, ids {ids.tolist()}", got_is_bf16=True)
+
+
 @pytest.mark.parametrize("name,T", [("c0", 1), ("c0", 6), ("c1", 1), ("c1", 2), ("c1", 3), ("c3_small", 1), ("c4", 2)])
 def test_flat_form_for_a_handful_of_slots(name, T):
     """Up to twelve routed slots the bf16 entry point runs two flat kernels (moe_gemv.cu) instead

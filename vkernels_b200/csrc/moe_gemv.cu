@@ -246,18 +246,16 @@ gemv_down_kernel(const uint16_t* __restrict__ act, const uint8_t* __restrict__ w
   if (tid < 16) {
     const int h = h0 + tid;
     float acc = 0.0f;
-    int last = -1;   // slots in ascending expert order (a token's experts are distinct)
+    int last = -1;   // slots in ascending order of the expert, a repeated expert's in their own
     for (int n = 0; n < top_k; ++n) {
-      int best = -1, best_e = 0x7FFFFFFF;
+      int best_key = 0x7FFFFFFF;
       for (int jj = 0; jj < top_k; ++jj) {
-        const int ee = s_e[jj];
-        if (ee > last && ee < best_e) {
-          best_e = ee;
-          best = jj;
-        }
+        const int key = s_e[jj] * kTinyMaxSlots + jj;   // (below 0 for a skipped slot)
+        if (key > last && key < best_key) best_key = key;
       }
-      if (best < 0) break;
-      last = best_e;
+      if (best_key == 0x7FFFFFFF) break;
+      last = best_key;
+      const int best_e = best_key / kTinyMaxSlots, best = best_key - best_e * kTinyMaxSlots;
       float v = 0.0f;
 #pragma unroll
       for (int p = 0; p < KSPLIT; ++p) v += part[best][p][tid];
