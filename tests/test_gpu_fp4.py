@@ -103,28 +103,59 @@ def test_longest_reductions(H, I):
     assert np.linalg.norm(got - ref) <= 2.0 ** -8 * np.linalg.norm(ref)   # (the bound of test_tile_edges)
 
 
-def test_wide_range_rows():
-    """Rows whose elements span far more than the seventeen bits of their integers, and rows near both ends of the
-    bf16 range: the error stays below 2^-17 of the row's largest element times the weights' 1-norm."""
-    H, I, counts = 256, 64, (5, 20, 16)
-    w, A, ids, tw = _problem(H, I, counts)
-    T = A.shape[0]
-    g = torch.Generator(device=DEV)
-    g.manual_seed(1)
-    A *= torch.exp2(torch.randint(-24, 1, A.shape, generator=g, device=DEV).float()).to(torch.bfloat16)
-    A *= torch.exp2(torch.linspace(-120, 20, T, device=DEV)).to(torch.bfloat16)[:, None]
-    sids, eids, _ = ops.moe_align_block_size(ids, len(counts), 16)
-    act = torch.zeros((sids.numel(), I), dtype=torch.bfloat16, device=DEV)
+def _one_hot(rows, K, first=0):
+    """[rows, K / 2] codes: row first + k holds a 1 (code 2) at k, everything else is zero."""
+    codes = np.zeros((rows, K), np.uint8)
+    codes[first + np.arange(K), np.arange(K)] = 2
+    return codes[:, 0::2] | (codes[:, 1::2] << 4)
+
+
+@pytest.mark.parametrize("lead", [(-133, -120), (-20, 20), (100, 121)])
+def test_digit_planes_of_wide_range_rows(lead):
+    """Both GEMMs made the identity (one-hot weights, a gate of 64 from its bias), so that what comes out is the token operand as
+    its digit planes hold it: elements down to 2^-9 of the row's leading power of two exactly, smaller ones to half a unit of the
+    integers, 2^-17 of it - in rows of subnormals, ordinary rows and rows up to the end of the bf16 range."""
+    H = I = 256
+    counts = (5, 20, 16)
+    E, T = len(counts), sum(counts)
+    w = {"w13": torch.from_numpy(np.stack([_one_hot(2 * I, H, I)] * E)).to(DEV), "w2": torch.from_numpy(np.stack([_one_hot(H, I)] * E)).to(DEV),
+         "w13_scale": torch.full((E, 2 * I, H // 32), 127, dtype=torch.uint8, device=DEV),
+         "w2_scale": torch.full((E, H, I // 32), 127, dtype=torch.uint8, device=DEV)}
+    b13 = torch.zeros((E, 2 * I), device=DEV)
+    b13[:, :I] = 64.0
+    rng = np.random.default_rng(4)
+    x = (1 + rng.integers(0, 128, (T, H)) / 128.0) * rng.choice([-1.0, 1.0], (T, H)) * 2.0 ** -rng.integers(0, 25, (T, H)).astype(np.float64)
+    x[:, 7] = 1.5
+    x *= 2.0 ** np.linspace(*lead, T).round()[:, None]
+    A = torch.from_numpy(x).to(DEV).to(torch.bfloat16)
+    ids = torch.from_numpy(rng.permutation(np.repeat(np.arange(E), counts)).astype(np.int32)[:, None]).to(DEV)
+    tw = torch.ones((T, 1), device=DEV)
+
+    def check(got, operand, gain, rounding, what, smallest=0.0):
+        power = torch.exp2(torch.floor(torch.log2(operand.abs().amax(1, keepdim=True))))
+        want = gain * operand
+        exact = (operand.abs() >= power * 2.0 ** -9) & (want.abs() >= smallest)
+        assert (operand != 0).any(1).all() and exact.any(1).all() and (lead[0] < -126 or not exact.all(1).any())
+        assert torch.equal(got[exact], want[exact]), what
+        # a bf16 result adds half a step of itself, or of the smallest subnormal
+        bound = gain * power * 2.0 ** -17 + rounding * (2.0 ** -8 * want.abs() + 2.0 ** -134)
+        assert ((got - want).abs() <= bound + torch.where(want.abs() < smallest, want.abs(), 0.0)).all(), what
+
+    out, act, sids, _, _ = gpu_layer(A, w, ids, tw, b13=b13, return_parts=True)
+    rows = torch.empty(T, dtype=torch.long, device=DEV)
+    real = ((sids >= 0) & (sids < T)).nonzero().flatten()
+    rows[sids[real].long()] = real
+    act = act[rows].double()
+    check(act, A.double(), 64.0, 1, "gate/up")
+    check(out.double(), act, 1.0, 0, "down", smallest=2.0 ** -126)   # (red.global.add.f32 takes subnormals as zeros)
+    sids, eids, _ = ops.moe_align_block_size(ids, E, 16)
+    pk = ops.prepack_weights(w["w13"], w["w13_scale"], w["w2"], w["w2_scale"])
+    act_p = torch.zeros((sids.numel(), I), dtype=torch.bfloat16, device=DEV)
     y = torch.empty((T, H), dtype=torch.bfloat16, device=DEV)
-    # SiTU with huge beta's is close to the identity on small inputs; large ones saturate: only the gate sums matter here,
-    # so compare the activations with those of the CUDA-core path
-    ops.fused_moe_mxfp4_bf16_into(y, act, A, w["w13"], w["w13_scale"], w["w2"], w["w2_scale"], tw.reshape(-1), sids, eids, top_k=1)
-    _, ref, _, _, _ = gpu_layer(A, w, ids, tw, impl="simt", return_parts=True)
-    real = (sids >= 0) & (sids < T)
-    a, r = act[real].double(), ref[real].double()
-    # relative to the row: activations are about u * g / 2 with both linear in the row's scale
-    scale = r.abs().amax(1, keepdim=True).clamp_min(1e-300)
-    assert ((a - r).abs() / scale).max().item() <= 2.0 ** -7
+    ops.fused_moe_mxfp4_bf16_prepacked_into(y, act_p, A, pk, tw.reshape(-1), sids, eids, top_k=1, b13=b13)
+    torch.cuda.synchronize()
+    assert torch.equal(act_p[rows].double(), act)
+    check(y.double(), act, 1.0, 1, "down, prepacked")
 
 
 @pytest.mark.parametrize("code", [0x6, 0xE, 0x7])
