@@ -29,9 +29,9 @@
 //
 // Batches of up to a few dozen tokens an expert run moe_gemm_fp4.cu instead. Two forms here, chosen by the largest token
 // tile of the launch:
-//   lone CTA (tiles up to 128 tokens, and the stage split of tensor parallelism): the stage length grows as the tile
-//     shrinks (256 K-elements up to 64 tokens, 128 up to 128), because the issuer's per-stage
-//     handshake costs a few hundred cycles whatever the stage holds;
+//   lone CTA (the stage split of tensor parallelism, VK_MOE_SMALL=bf16, VK_MOE_PAIR=0, and reductions too long for a
+//     pair): stages of 256 K-elements for tiles of up to 64 tokens, because the issuer's per-stage
+//     handshake costs a few hundred cycles whatever the stage holds, and of 64 for tiles of up to 256;
 //   CTA pair (larger tiles, the prefill regime): a cluster of two CTAs works on one item of
 //     256 weight rows x up to 320 tokens with cta_group::2 MMAs. Each CTA dequantises its own
 //     128 rows and stages HALF of the token rows, which halves the token bytes an SM pulls
@@ -137,7 +137,7 @@ struct GemmParams {
 // ---------------------------------------------------------------------------
 // Accumulator columns: a lone CTA sizes them by the stage length (long stages serve small token
 // tiles), a pair always holds up to kPairMaxTok tokens.
-constexpr int acc_cols(int ks, int ctas) { return ctas == 2 ? kPairMaxTok : (ks == 64 ? 256 : (ks == 128 ? 128 : 64)); }
+constexpr int acc_cols(int ks, int ctas) { return ctas == 2 ? kPairMaxTok : (ks == 64 ? 256 : 64); }
 
 struct Barriers {
   uint64_t w_full[kMaxWStages], w_empty[kMaxWStages];
@@ -169,7 +169,7 @@ struct TokMaps {
 // slot in shared memory, one handshake of the MMA issuer). The issuer's
 // per-stage latency (barrier polls + commit) is a few hundred cycles whatever
 // the stage holds, so small token tiles, whose MMAs are short, take long
-// stages: KS = 64 for tiles up to 256 tokens, 128 up to 128, 256 up to 64.
+// stages: lone CTA, KS = 64 for tiles up to 256 tokens, 256 up to 64; pair, KS = 128.
 template <bool GATEUP, int KS, int CTAS>
 __global__ void __launch_bounds__(block_threads(CTAS), 1)
 moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
@@ -177,7 +177,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_w,
   constexpr int kThreads = block_threads(CTAS);
   constexpr int kAccCols = acc_cols(KS, CTAS);
   constexpr int kACols = KS / 2;                                      // columns of one A slot
-  constexpr int kAStages = (kTmemCols - kAccCols) / kACols;           // lone CTA: 8, 6, 3; pair: 6, 3
+  constexpr int kAStages = (kTmemCols - kAccCols) / kACols;           // lone CTA: 3 of 256, 8 of 64; pair: 3 of 128
   constexpr int kSubPerW = kWStageK / KS;                             // stages per packed-weight stage
   constexpr int kPieces = KS / 64;                                    // 64-K pieces of a stage
   static_assert(kAStages <= kMaxAStages, "A ring too deep for the barrier arrays");
@@ -1242,12 +1242,12 @@ void launch_gemm_ks(const CUtensorMap& tw, const TokMaps& tb, GemmParams p,
   }
 }
 
-// Stage length and CTA grouping by the largest token tile of the launch (see the kernel's comment).
+// Stage length and CTA grouping by the largest token tile of the launch (see the kernel's comment; choose_tiles makes none of
+// 65 to 128 tokens).
 template <bool GATEUP>
 void launch_gemm(const CUtensorMap& tw, const TokMaps& tb, GemmParams p,
                  bool use_pair, cudaStream_t stream) {
   if (p.max_tok <= 64) launch_gemm_ks<GATEUP, 256, 1>(tw, tb, p, stream);
-  else if (p.max_tok <= 128) launch_gemm_ks<GATEUP, 128, 1>(tw, tb, p, stream);
   else if (use_pair) launch_gemm_ks<GATEUP, 128, 2>(tw, tb, p, stream);
   else launch_gemm_ks<GATEUP, 64, 1>(tw, tb, p, stream);
 }
