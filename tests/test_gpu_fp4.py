@@ -59,6 +59,18 @@ def test_tile_edges(H, I, counts):
                 assert_close_bf16(y, ref, f"bf16 output {H} {I} {counts} {kw}", got_is_bf16=True)
 
 
+@pytest.mark.parametrize("H,I", [(512, 4096), (4096, 192), (4800, 2112), (192, 7168)])
+def test_several_items_a_cta(H, I):
+    """Experts of one and two tiles and more items than CTAs: a CTA goes on to another tile, or to another feature tile of the
+    same."""
+    w, A, ids, tw = _problem(H, I, (40, 33, 3, 0, 20, 50))
+    ref = oracle_layer(A, w, ids, tw)
+    got = to_np(gpu_layer(A, w, ids, tw))
+    assert np.linalg.norm(got - ref) <= 2.0 ** -8 * np.linalg.norm(ref)   # (the bound of test_tile_edges)
+    for y in _bf16_forms(w, A, ids, tw):                                  # (and half a step of the bf16 result)
+        assert np.linalg.norm(y - ref) <= (2.0 ** -8 + 2.0 ** -9) * np.linalg.norm(ref)
+
+
 @pytest.mark.parametrize("M,k,E", [(4, 4, 1), (8, 4, 2), (8, 8, 3), (5, 3, 2)])
 def test_an_expert_named_twice_by_a_token(M, k, E):
     """More rows in an expert than the batch has tokens: tiles of nine to sixteen rows, and several of them, in a batch of up

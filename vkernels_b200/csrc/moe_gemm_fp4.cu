@@ -23,8 +23,8 @@
 // prepacked 142 -> 117, 128 from the checkpoint layout 206 -> 152; 48 tokens of 16 experts each (hidden 7168, ispp
 // 512) 728 -> 400.
 //
-// Warp roles (one persistent CTA per SM; every CTA takes a contiguous range of the (token tile,
-// feature tile) items, so that the tile's rows and scales are looked up once for many items):
+// Warp roles (one persistent CTA per SM; the (token tile, feature tile) items are dealt out one after the
+// other):
 //   warp 0      TMA producer: packed weights (128 rows x 256 K a stage)
 //   warp 1      tcgen05.mma issuer + tensor-memory allocation
 //   warp 2      TMA producer: digit planes of the token tile
@@ -173,26 +173,34 @@ __device__ __noinline__ float nonfinite_part(const uint8_t* __restrict__ w, cons
   return sum;
 }
 
-// This CTA's walk over its contiguous share of the items; the tile is looked up when it changes.
+// This CTA's walk over its share of the items: every gridDim.x-th, so that the CTAs are at a few neighbouring tiles at any time
+// and their reads of a tile's planes (3 K bytes a token, once per feature tile), and of an expert's weights for its next tile, come
+// out of L2. With a contiguous range per CTA, which looks a tile up once for many items, the planes of as many tiles as there are CTAs
+// are in use beside the weight stream: 3760 us a layer at 1024 tokens of hidden 7168, ispp 2048, 256 + 1 experts for 3068 this way, 841 for
+// 748 at 1024 tokens of hidden = ispp = 2880 and 128 experts, 751 for 694 at 32 tokens of the wide shape prepacked; nowhere less. The tile is
+// looked up when it changes.
 struct Walk {
-  const TokTile* tiles;
-  int left, f, n_f, t;
+  const Fp4Params& p;
+  int left, f, t;
   TokTile tt;
-  __device__ __forceinline__ Walk(const TokTile* tiles_, int n_tiles, int n_f_) : tiles(tiles_), n_f(n_f_) {
-    const long long n = (long long)n_tiles * n_f;
-    const int lo = (int)(n * blockIdx.x / gridDim.x), hi = (int)(n * (blockIdx.x + 1) / gridDim.x);
-    left = hi - lo;
-    t = lo / n_f;
-    f = lo - t * n_f;
-    if (left > 0) tt = tiles[t];
+  __device__ __forceinline__ explicit Walk(const Fp4Params& p_) : p(p_) {
+    const long long n = (long long)*p.n_tiles * p.n_ftiles;
+    const int first = (int)blockIdx.x;
+    left = (int)((n - first + gridDim.x - 1) / gridDim.x);   // (not below 0: first < gridDim.x)
+    t = first / p.n_ftiles;
+    f = first - t * p.n_ftiles;
+    if (left > 0) tt = p.tiles[t];
   }
   __device__ __forceinline__ void next() {
     --left;
-    if (++f == n_f) {
-      f = 0;
+    const int was = t;
+    t += p.step_t;
+    f += p.step_f;
+    if (f >= p.n_ftiles) {
+      f -= p.n_ftiles;
       ++t;
-      if (left > 0) tt = tiles[t];
     }
+    if (t != was && left > 0) tt = p.tiles[t];
   }
 };
 // Tokens of a tile per MMA column block (8 or 16) and how many such blocks.
@@ -258,7 +266,7 @@ moe_gemm_fp4_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
   const int n_wrows = GATEUP ? 2 * p.n_feat : p.n_feat;
   const int n_kw = (p.K + kStageK - 1) / kStageK;
   const int pitch = p.K / 32;   // scale bytes per weight row
-  Walk wk(p.tiles, *p.n_tiles, p.n_ftiles);
+  Walk wk(p);
 
   if (warp == 0) {
     // ------------------- TMA producer: packed weights -----------------------
@@ -948,6 +956,8 @@ Fp4Plan fp4_plan(bool packed, int K, int tile_tok) {
 
 void launch_gemm_fp4(bool gateup, bool packed, Fp4Params p, const uint8_t* planes, int EM, cudaStream_t stream) {
   p.status = sm100_status_address();
+  p.step_t = sm_count() / p.n_ftiles;   // (the grid is one CTA per SM)
+  p.step_f = sm_count() % p.n_ftiles;
   const uint64_t half = (uint64_t)p.K / 2;
   const uint64_t xdims[3] = {half, (uint64_t)EM, kDigits}, xstr[2] = {half, half * EM};
   const uint32_t box8[3] = {128, 8, kDigits}, box16[3] = {128, 16, kDigits};

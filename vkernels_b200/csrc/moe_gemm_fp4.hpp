@@ -26,6 +26,7 @@ struct Fp4Params {
   int store_rows;             // with out_rows: slot j's unweighted row is stored at row j of the token's block
   int tile_tok;               // the tile list's limit (16 or 32): what a token slot holds
   int K, n_feat, n_ftiles;
+  int step_t, step_f;         // from one item of a CTA to its next (grid size items on) in tiles and feature tiles (launch_gemm_fp4)
   int N, top_k, w_sorted;
   int b_stages, b_stage_bytes, w_stages, scale_bufs, scale_buf_bytes, teams;   // (launch_gemm_fp4 fills these in)
   int activation;
