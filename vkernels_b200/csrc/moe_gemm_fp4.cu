@@ -11,17 +11,17 @@
 // padded form the copy engine can unpack to takes twice the shared memory and its bandwidth.
 //
 // kind::mxf4 wants four-bit tokens too. A bf16 row is written as x = s * v with s a power of two
-// and v a 17-bit integer (|v| < 2^17: exact unless an element lies more than 2^9 below the row's
-// largest, then off by at most 2^-18 of that largest value), and v as six balanced base-8 digits
+// and v a 17-bit integer (|v| < 2^17: exact unless an element lies more than 2^9 below the row's leading
+// power of two, then off by at most half a unit, 2^-17 of that power), and v as six balanced base-8 digits
 // -4..4, each of which is an e2m1 value. The six digit planes of a tile lie side by side along N:
 // an MMA of K = 64 takes 48 clocks at N = 96 and 96 at N = 192 (measured, the unit's full rate), its issue about 40, so
 // sixteen tokens cost little more than one. The epilogue adds the planes' sums, times 8^d s / 2, in fp32.
 //
 // What bounds it: the weight bytes. Per 128 rows x 256 K (17 KB) an SM gets its share of HBM in about 700 clocks. A
 // stage takes about 720 prepacked and 950 to 1000 from the checkpoint layout (the code warps' latency); with one byte a
-// weight it took 1100 and 1700. Whole decode steps of the gpt-oss-20b shape: 8 tokens prepacked 105 -> 87 us, 64
-// prepacked 142 -> 117, 128 from the checkpoint layout 206 -> 152; 48 tokens of 16 experts each (hidden 7168, ispp
-// 512) 728 -> 400.
+// weight it took 1100 and 1700. Whole decode steps of the gpt-oss-20b shape: 8 tokens prepacked 105 -> 84 us, 64
+// prepacked 142 -> 117, 128 from the checkpoint layout 203 -> 148; 48 tokens of 16 experts each (hidden 7168, ispp
+// 512) 719 -> 379.
 //
 // Warp roles (one persistent CTA per SM; the (token tile, feature tile) items are dealt out one after the
 // other):

@@ -1413,7 +1413,8 @@ TileChoice choose_tiles(int M, int top_k, int EM, int block_size, int k_gateup, 
   max_tok = ((max_tok + 15) / 16) * 16;
   // When an expert sees a few dozen tokens at most, tiles are capped at 64 rows so that the launch
   // takes the long-stage form built for small tiles (an expert with more rows is split into
-  // several items); measured crossover against the CTA-pair form: about 48 tokens per expert.
+  // several items); the crossover against the CTA-pair form, about 48 tokens per expert, was measured with the byte form that
+  // ran small tiles before the fp4 form.
   {
     const long long n_slots = (long long)M * top_k;
     if ((M <= 256 || n_slots <= 48 * experts_estimate(M, top_k, EM, block_size)) && max_tok > 64) max_tok = 64;
